@@ -137,8 +137,11 @@ struct fdtd_solver {
     std::vector<uint32_t> layer_cells;      // pitched, in the layout's order (for fdtd_read_state)
     const uint8_t *types_device = nullptr;  // the pitched cell types
     const float *scale_device = nullptr;    // with a speed field: each pitched cell's scale
-    // The matched layer's state (kLayerSlots values a pitched cell: its parts and the velocities on
-    // its + faces; only the layer's cells and their - faces used), in two buffers: layer_state[1]
+    // The matched layer's quads (Tables) and each layer cell's lane, on the host (for
+    // fdtd_read_state).
+    std::vector<uint4> layer_quads;
+    std::vector<uint32_t> layer_lane;
+    // The matched layer's state (kLayerSlots slots of layer_lanes values), in two buffers: layer_state[1]
     // holds the latest values between runs, as u[1] does.
     void *layer_state[2] = {nullptr, nullptr};
     uint32_t link_slots = 0;  // the most links of a special row (6 or 18 kernels)
@@ -692,7 +695,7 @@ int launch_steps(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
     const uint64_t layer_cap = s->layer_per_sm ? (uint64_t)s->sms * s->layer_per_sm : UINT64_MAX;
     const uint32_t special_blocks = (uint32_t)std::min<uint64_t>((s->specials + kBlock - 1) / kBlock, special_cap);
     const uint32_t probe_blocks = (uint32_t)((s->probes + kProbeWarps - 1) / kProbeWarps);
-    const uint32_t layer_blocks = (uint32_t)std::min<uint64_t>((s->layers + kBlock - 1) / kBlock, layer_cap);
+    const uint32_t layer_blocks = (uint32_t)std::min<uint64_t>((g.layer_quads + kBlock - 1) / kBlock, layer_cap);
     // Each step: the interior sweep on the handle's stream; beside it the matched layer on the
     // layer stream, of the highest priority (its blocks take the thread slots that the sweep's
     // shared memory leaves free on every multiprocessor), and the special rows and probes on the
@@ -1017,9 +1020,6 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
         if ((rc = zeros(s, e * L->state_count, &s->w[k]))) return rc;
     }
     if (s->precision == FDTD_FP32_COMPENSATED && (rc = zeros(s, e * s->n_device, &s->increment))) return rc;
-    if (L->layer_count)
-        for (int k = 0; k < 2; ++k)
-            if ((rc = zeros(s, e * kLayerSlots * s->n_device, &s->layer_state[k]))) return rc;
     void *flag;
     if ((rc = zeros(s, sizeof(unsigned int), &flag))) return rc;
     s->d_error = static_cast<unsigned int *>(flag);
@@ -1158,31 +1158,57 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
     if (Lc) {
         std::vector<uint32_t> cells(Lc);
         for (uint64_t c = 0; c < Lc; ++c) cells[c] = pitched(s, (uint64_t)L->layer_cells[c]);
-        // Which of each layer cell's lower neighbours are in the layer too (their face is theirs).
-        std::vector<uint8_t> below(Lc, 0);
-        const uint64_t strides[3] = {1, nx, nx * ny};
-        for (uint64_t c = 0; c < Lc; ++c)
-            for (int axis = 0; axis < 3; ++axis)
-                if (L->types[(uint64_t)L->layer_cells[c] - strides[axis]] == kLayer) below[c] |= (uint8_t)(1u << axis);
         s->layer_cells = cells;
         const uint32_t *p;
         if ((rc = upload(s, cells.data(), Lc, &p))) return rc;
         g.layer_cells = p;
-        if ((rc = upload(s, below.data(), Lc, &u8))) return rc;
-        g.layer_below = u8;
+        // The quads that hold layer cells, or the cells below them, in the grid's order.
+        std::vector<uint32_t> quad_of(s->n_device / 4, UINT32_MAX);
+        const uint32_t strides[3] = {1, g.pitch, g.plane};
+        for (const uint32_t i : cells) {
+            quad_of[i / 4] = 0;
+            for (const uint32_t stride : strides) quad_of[(i - stride) / 4] = 0;
+        }
+        std::vector<uint4> &quads = s->layer_quads;
+        for (uint64_t q = 0; q < quad_of.size(); ++q)
+            if (!quad_of[q]) quad_of[q] = (uint32_t)quads.size(), quads.push_back(make_uint4((uint32_t)(4 * q), 0, 0, 0));
+        if (quads.size() >= (1ull << 30)) return fail(s, FDTD_EINVAL, "the matched layer is too large for the GPU's 32-bit indices");
+        std::vector<uint32_t> lane_cell(4 * quads.size(), 0);
+        s->layer_lane.resize(Lc);
+        for (uint64_t c = 0; c < Lc; ++c) {
+            const uint32_t i = cells[c], q = quad_of[i / 4], j = i % 4;
+            uint4 &entry = quads[q];
+            entry.y = quad_of[(i - strides[1]) / 4], entry.z = quad_of[(i - strides[2]) / 4];
+            entry.w |= 1u << j;
+            const uint64_t l = (uint64_t)L->layer_cells[c], below[3] = {1, nx, nx * ny};
+            for (int axis = 0; axis < 3; ++axis)
+                if (L->types[l - below[axis]] == kLayer) entry.w |= 1u << (4 + 4 * axis + j);
+            s->layer_lane[c] = 4 * q + j;
+            lane_cell[4 * (uint64_t)q + j] = (uint32_t)c;
+        }
+        g.layer_quads = (uint32_t)quads.size(), g.layer_lanes = 4 * g.layer_quads;
+        if ((rc = upload(s, quads.data(), quads.size(), &g.layer_quad))) return rc;
+        if ((rc = upload(s, lane_cell.data(), lane_cell.size(), &g.lane_cell))) return rc;
+        for (int k = 0; k < 2; ++k)
+            if ((rc = zeros(s, e * kLayerSlots * g.layer_lanes, &s->layer_state[k]))) return rc;
         const uint64_t len[3] = {nx + 1, ny + 1, nz + 1};
         for (int axis = 0; axis < 3; ++axis) {
-            std::vector<float4> packed(len[axis]);
+            // (Along x padded to the pitch: a quad's lanes beyond the grid read entries too.)
+            std::vector<float4> packed(axis == 0 ? s->pitch + 2 : len[axis], make_float4(0.0f, 0.0f, 0.0f, 0.0f));
             for (uint64_t x = 0; x < len[axis]; ++x)
                 packed[x] = make_float4(L->keep[2 * axis][x], L->push[2 * axis][x], L->keep[2 * axis + 1][x],
                                         L->push[2 * axis + 1][x]);
             const float4 *p4;
-            if ((rc = upload(s, packed.data(), len[axis], &p4))) return rc;
+            if ((rc = upload(s, packed.data(), packed.size(), &p4))) return rc;
             g.layer_coef[axis] = p4;
         }
         if (s->scaled) {
             if ((rc = upload(s, L->layer_scale, Lc, &fp))) return rc;
             g.layer_scale = fp;
+            std::vector<float> lane_scale(g.layer_lanes, 1.0f);
+            for (uint64_t c = 0; c < Lc; ++c) lane_scale[s->layer_lane[c]] = L->layer_scale[c];
+            if ((rc = upload(s, lane_scale.data(), lane_scale.size(), &fp))) return rc;
+            g.lane_scale = fp;
         }
     }
 
@@ -1658,7 +1684,7 @@ struct Kept {
 uint64_t checkpoint_bytes(const fdtd_solver *s) {
     const uint64_t e = s->precision == FDTD_FP64 ? 8 : 4;
     uint64_t bytes = 2 * e * s->n_device + 2 * e * s->states;
-    if (s->layers) bytes += kLayerSlots * e * s->n_device;
+    bytes += kLayerSlots * e * s->tables.layer_lanes;
     return bytes;
 }
 
@@ -1672,7 +1698,7 @@ int save_checkpoint(fdtd_solver *s, char *c) {
         CUDA_TRY(s, cudaMemcpyAsync(c + states, s->w[0], states, cudaMemcpyDeviceToDevice, s->stream));
     }
     c += 2 * states;
-    if (s->layers) CUDA_TRY(s, cudaMemcpyAsync(c, s->layer_state[1], kLayerSlots * level, cudaMemcpyDeviceToDevice, s->stream));
+    if (s->layers) CUDA_TRY(s, cudaMemcpyAsync(c, s->layer_state[1], kLayerSlots * e * s->tables.layer_lanes, cudaMemcpyDeviceToDevice, s->stream));
     return FDTD_OK;
 }
 
@@ -1686,7 +1712,7 @@ int restore_checkpoint(fdtd_solver *s, const char *c) {
         CUDA_TRY(s, cudaMemcpyAsync(s->w[0], c + states, states, cudaMemcpyDeviceToDevice, s->stream));
     }
     c += 2 * states;
-    if (s->layers) CUDA_TRY(s, cudaMemcpyAsync(s->layer_state[1], c, kLayerSlots * level, cudaMemcpyDeviceToDevice, s->stream));
+    if (s->layers) CUDA_TRY(s, cudaMemcpyAsync(s->layer_state[1], c, kLayerSlots * e * s->tables.layer_lanes, cudaMemcpyDeviceToDevice, s->stream));
     return FDTD_OK;
 }
 
@@ -3061,7 +3087,7 @@ int fdtd_reset(fdtd_solver *s) {
     }
     if (s->increment) CUDA_TRY(s, cudaMemsetAsync(s->increment, 0, e * s->n_device, s->stream));
     if (s->layers)
-        for (int k = 0; k < 2; ++k) CUDA_TRY(s, cudaMemsetAsync(s->layer_state[k], 0, e * kLayerSlots * s->n_device, s->stream));
+        for (int k = 0; k < 2; ++k) CUDA_TRY(s, cudaMemsetAsync(s->layer_state[k], 0, e * kLayerSlots * s->tables.layer_lanes, s->stream));
     CUDA_TRY(s, cudaStreamSynchronize(s->stream));
     s->steps_done = 0;
     return FDTD_OK;
@@ -3123,18 +3149,18 @@ int fdtd_read_state(const fdtd_solver *cs, void *current, void *previous, void *
     if (layer_state && s->layers) {
         // The reference's nine values per cell (fdtd.hpp:2245): the parts, then per axis the
         // velocity of the - face (the + face of the cell below) and of the + face.
-        const std::vector<uint32_t> &cells = s->layer_cells;
-        std::vector<char> state(e * kLayerSlots * s->n_device);
+        const uint64_t lanes = s->tables.layer_lanes;
+        std::vector<char> state(e * kLayerSlots * lanes);
         CUDA_TRY(s, cudaMemcpy(state.data(), s->layer_state[1], state.size(), cudaMemcpyDeviceToHost));
         char *dst = static_cast<char *>(layer_state);
-        const uint64_t strides[3] = {1, s->pitch, s->pitch * s->ny};
         for (uint64_t c = 0; c < s->layers; ++c) {
-            const uint64_t i = cells[c];
-            for (int k = 0; k < 3; ++k) std::memcpy(dst + e * (9 * c + k), state.data() + e * (kLayerSlots * i + k), e);
-            for (int axis = 0; axis < 3; ++axis) {
-                const uint64_t below = kLayerSlots * (i - strides[axis]) + 3 + axis, own = kLayerSlots * i + 3 + axis;
-                std::memcpy(dst + e * (9 * c + 3 + 2 * axis), state.data() + e * below, e);
-                std::memcpy(dst + e * (9 * c + 4 + 2 * axis), state.data() + e * own, e);
+            const uint64_t own = s->layer_lane[c], j = own % 4;
+            const uint4 &quad = s->layer_quads[own / 4];
+            const uint64_t below[3] = {own - 1, 4 * (uint64_t)quad.y + j, 4 * (uint64_t)quad.z + j};
+            for (uint64_t k = 0; k < 3; ++k) std::memcpy(dst + e * (9 * c + k), state.data() + e * (k * lanes + own), e);
+            for (uint64_t axis = 0; axis < 3; ++axis) {
+                std::memcpy(dst + e * (9 * c + 3 + 2 * axis), state.data() + e * ((3 + axis) * lanes + below[axis]), e);
+                std::memcpy(dst + e * (9 * c + 4 + 2 * axis), state.data() + e * ((3 + axis) * lanes + own), e);
             }
         }
     }

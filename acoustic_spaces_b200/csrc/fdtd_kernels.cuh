@@ -33,9 +33,8 @@ namespace fdtd {
 
 constexpr int kSolid = 0, kInterior = 1, kSpecial = 2, kLayer = 3;
 constexpr int kBlock = 128;  // threads per block of every kernel
-// A matched-layer cell's state — its three pressure parts and the velocities on its three + faces —
-// sits together, six values a cell in a pitched array (two such arrays, the state a step before and
-// the new one): one stream of memory for the state in place of nine.
+// A matched-layer cell's state: its three pressure parts and the velocities on its three + faces (two
+// such sets, the state a step before and the new one).
 constexpr int kLayerSlots = 6;
 
 // ---- the bulk sweep's tiles ------------------------------------------------------------------
@@ -525,7 +524,16 @@ struct Tables {
     const uint32_t *layer_cells;
     const float *layer_scale;
     const float4 *layer_coef[3];
-    const uint8_t *layer_below;  // bit a: the cell below along axis a is in the layer too
+    // The quads that hold layer cells or cells below one (four adjacent cells of a row each, from a
+    // multiple of four; ascending): {the quad's pitched index, the quads a row and a plane before it,
+    // bits 0-3: its layer cells, bits 4 a + 4 ..: those whose cell below along axis a is in the layer
+    // too}. The quad before along x, where a cell of it is read, is the one before in the list.
+    // layer_lanes: four a quad, the length of a state slot; each lane's layer cell, and with a speed
+    // field its scale.
+    uint32_t layer_quads, layer_lanes;
+    const uint4 *layer_quad;
+    const uint32_t *lane_cell;
+    const float *lane_scale;
     uint32_t plane;  // pitch * ny
     FastDiv by_plane, by_pitch;  // a pitched index's plane, and its row within the plane
     // With a tangent of the layer's tables (fdtd_set_layer_tangent): per axis and coordinate the
@@ -548,9 +556,9 @@ struct Fields {
     const T *b;        // the current pressure
     T *wa;             // branch velocities a step before, overwritten with the next
     const T *wb;       // current branch velocities
-    // The matched layer's state, kLayerSlots values a (pitched) cell: at kLayerSlots i + axis the
-    // layer cell's pressure part along that axis, at kLayerSlots i + 3 + axis the velocity on its
-    // + face along it (also kept at a cell outside the layer whose + face is a layer cell's - face).
+    // The matched layer's state by slot and lane: slot a the pressure part along axis a, slot 3 + a the
+    // velocity on the + face along it (also kept at a cell outside the layer whose + face is a layer
+    // cell's - face), lane 4 q + j cell j of quad q.
     const T *cell_old;  // a step before
     T *cell_new;        // this step
     const float *signal;  // the step's drive at signal[0]
@@ -576,11 +584,25 @@ struct Fields {
 // The links' tables are read once a step and the new pressure by no kernel of the same step, so
 // those go through the caches as streaming (evict-first) accesses, leaving L2 to the pressures
 // that the sweep and the layer share with the rows (measured: the concurrent step 2 % shorter).
-template <typename T, int SLOTS, bool COMP>
+// (The resident stepper, whose tables and levels stay in L2 between steps, takes them as plain
+// accesses: STREAM false.)
+template <bool STREAM, typename V>
+__device__ __forceinline__ V load_once(const V *p) {
+    return STREAM ? __ldcs(p) : *p;
+}
+template <bool STREAM, typename V>
+__device__ __forceinline__ void store_once(V *p, V value) {
+    if (STREAM)
+        __stcs(p, value);
+    else
+        *p = value;
+}
+
+template <typename T, int SLOTS, bool COMP, bool STREAM = true>
 __device__ __forceinline__ void special_row(const Tables &g, const Fields<T> &f, const uint32_t k, const uint32_t i,
                                             const uint32_t links, const uint32_t s0, const uint32_t s1) {
     const uint32_t K = g.specials;
-    const T *__restrict__ b = f.b;
+    const T *b = f.b;
     T sum = 0;
     T here;
     if constexpr (SLOTS == 0) {
@@ -603,8 +625,8 @@ __device__ __forceinline__ void special_row(const Tables &g, const Fields<T> &f,
             weight[l] = 0.0f;
             if ((uint32_t)l < links) {
                 const uint32_t at = l * K + k;
-                weight[l] = __ldcs(g.link_weight + at);
-                value[l] = b[(uint32_t)((int64_t)i + g.offset[__ldcs(g.link_direction + at)])];
+                weight[l] = load_once<STREAM>(g.link_weight + at);
+                value[l] = b[(uint32_t)((int64_t)i + g.offset[load_once<STREAM>(g.link_direction + at)])];
             }
         }
         here = b[i];
@@ -632,7 +654,7 @@ __device__ __forceinline__ void special_row(const Tables &g, const Fields<T> &f,
     const T previous = f.a[i];
     const T next = ((T)g.coef_a[k] * here + sum - (T)g.coef_b[k] * previous - flow +
                     (T)g.source[k] * (T)f.signal[0]) * (T)g.coef_inv[k];
-    __stcs(f.a + i, next);
+    store_once<STREAM>(f.a + i, next);
     if (f.traj_u) f.traj_u[k] = next;
     for (uint32_t j = s0; j < s1; ++j) {
         const T own = (T)g.state_now[j] * f.wb[j] - (T)g.state_before[j] * f.wa[j];
@@ -665,126 +687,204 @@ __global__ void __launch_bounds__(kBlock) special_kernel(const Tables g, const F
     }
 }
 
-// Matched-layer cells (fdtd.hpp:2242-2264), one a thread: per axis the cell's two face
+// Four adjacent cells of a row, at a multiple of four cells (16-byte aligned).
+template <typename T>
+struct Quad {
+    T v[4];
+};
+
+__device__ __forceinline__ Quad<float> load_quad(const float *p) {
+    const float4 a = *reinterpret_cast<const float4 *>(p);
+    return {{a.x, a.y, a.z, a.w}};
+}
+__device__ __forceinline__ Quad<double> load_quad(const double *p) {
+    const double2 a = *reinterpret_cast<const double2 *>(p), b = *reinterpret_cast<const double2 *>(p + 2);
+    return {{a.x, a.y, b.x, b.y}};
+}
+template <bool STREAM>
+__device__ __forceinline__ void store_quad(float *p, const Quad<float> &q) {
+    store_once<STREAM>(reinterpret_cast<float4 *>(p), make_float4(q.v[0], q.v[1], q.v[2], q.v[3]));
+}
+template <bool STREAM>
+__device__ __forceinline__ void store_quad(double *p, const Quad<double> &q) {
+    store_once<STREAM>(reinterpret_cast<double2 *>(p), make_double2(q.v[0], q.v[1]));
+    store_once<STREAM>(reinterpret_cast<double2 *>(p + 2), make_double2(q.v[2], q.v[3]));
+}
+// The cells of `mask` (bit j: cell j) stored, as one vector where all four are.
+template <bool STREAM, typename T>
+__device__ __forceinline__ void store_cells(T *p, const Quad<T> &q, uint32_t mask) {
+    if (mask == 15u) {
+        store_quad<STREAM>(p, q);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (mask & (1u << j)) store_once<STREAM>(p + j, q.v[j]);
+    }
+}
+
+// A quad of scales as T (1 without a speed field).
+template <typename T, bool SCALED>
+__device__ __forceinline__ Quad<T> scales(const float *scale, uint32_t i) {
+    if (!SCALED) return {{(T)1, (T)1, (T)1, (T)1}};
+    const float4 s = __ldg(reinterpret_cast<const float4 *>(scale + i));
+    return {{(T)s.x, (T)s.y, (T)s.z, (T)s.w}};
+}
+
+// Matched-layer cells (fdtd.hpp:2242-2264), a quad of them a thread: per axis each cell's two face
 // velocities, then its pressure part; the cell's pressure is the parts' sum.
 //
 // The reference keeps, per layer cell, its own copy of the velocity on each of its six faces
 // (fdtd.hpp:2245), and both cells of a face update their copies alike: cell i's + face along an
 // axis of stride s and cell i+s's - face take keep_face[x+1] * u - push_face[x+1] * (b[i+s] -
 // b[i]) from the same value, so that, both starting at 0, the two copies stay equal to the bit.
-// Here each face is kept once, on the cell below it (face[i] is cell i's + face), in two buffers
-// that alternate with the steps: every cell reads the old values of its two faces and works both
-// out again, and writes the new value of its + face, and of its - face too where the cell below
-// is not in the layer (no one else writes that face). The pressure parts stay per cell.
-template <typename T, bool SCALED, bool COMP>
-__device__ __forceinline__ void layer_cell(const Tables &g, const Fields<T> &f, const uint32_t c, const uint32_t i) {
-    const uint32_t L = g.layers;
-    // Every load of the cell first — its parts, its pressure and its six neighbours', its faces'
-    // old velocities and the coefficients — so that they are in flight together; then the
-    // reference's arithmetic, axis by axis; then the stores, as streaming (evict-first) stores:
-    // the new state and pressure are read by no kernel of the same step.
-    const uint32_t z = g.by_plane(i), r = i - z * g.plane, y = g.by_pitch(r);
-    const uint32_t at[3] = {r - y * g.pitch, y, z};
-    const uint32_t strides[3] = {1u, g.pitch, g.plane};
-    const T *__restrict__ b = f.b;
-    using V2 = typename Pair<T>::type;
-    T part[3], lo[3], hi[3], old_below[3], old_above[3];
-    float4 c0[3], c1[3];
-    {
-        // the cell's own state in three vector loads: parts x, y; part z, face x; faces y, z
-        const V2 *own = reinterpret_cast<const V2 *>(f.cell_old + (uint64_t)kLayerSlots * i);
-        const V2 s0 = own[0], s1 = own[1], s2 = own[2];
-        part[0] = s0.x, part[1] = s0.y, part[2] = s1.x;
-        old_above[0] = s1.y, old_above[1] = s2.x, old_above[2] = s2.y;
-    }
+// Here each face is kept once, on the cell below it, in two buffers that alternate with the steps:
+// every cell reads the old values of its two faces and works both out again, and writes the new
+// value of its + face, and of its - face too where the cell below is not in the layer (no one else
+// writes that face). The pressure parts stay per cell.
+//
+// The state lies by slot and quad rather than by cell of the grid, so that a warp's accesses are
+// whole lines of 16 bytes a lane: the six slots, the faces below along y and z, the pressures and
+// their neighbours take some twenty vector loads for four cells in place of eighteen scattered
+// ones a cell.
+template <typename T>
+struct LayerState {
+    Quad<T> part[3], lo[3], hi[3];  // per axis: the parts, the - faces' velocities, the + faces'
+};
+
+// A quad's state as the slots hold it: its own six, and the - faces from the quads below.
+template <typename T>
+__device__ __forceinline__ void load_layer(const T *old, const uint64_t lanes, const uint32_t q, const uint4 d, LayerState<T> &s) {
 #pragma unroll
-    for (int axis = 0; axis < 3; ++axis) {
-        const uint32_t stride = strides[axis];
-        lo[axis] = b[i - stride];
-        hi[axis] = b[i + stride];
-        old_below[axis] = f.cell_old[(uint64_t)kLayerSlots * (i - stride) + 3 + axis];
-        c0[axis] = __ldg(g.layer_coef[axis] + at[axis]);
-        c1[axis] = __ldg(g.layer_coef[axis] + at[axis] + 1);
+    for (int a = 0; a < 3; ++a) {
+        s.part[a] = load_quad(old + a * lanes + 4 * (uint64_t)q);
+        s.hi[a] = load_quad(old + (3 + a) * lanes + 4 * (uint64_t)q);
     }
-    const T here = b[i];
-    const T scale = SCALED ? (T)g.layer_scale[c] : (T)1;
-    const uint32_t shared_below = g.layer_below[c];
-    const uint32_t tangent_axes = f.traj_tangent ? g.tangent_axes[c] : 0u;
-    uint32_t tangent_slot = f.traj_tangent ? g.tangent_start[c] : 0u;
-    T below[3], above[3];
-    T total = 0;
+    s.lo[0].v[0] = (d.w & 1u) ? old[3 * lanes + 4 * (uint64_t)q - 1] : (T)0;
 #pragma unroll
-    for (int axis = 0; axis < 3; ++axis) {
-        below[axis] = (T)c0[axis].z * old_below[axis] - (T)c0[axis].w * (here - lo[axis]);
-        above[axis] = (T)c1[axis].z * old_above[axis] - (T)c1[axis].w * (hi[axis] - here);
-        if (COMP) {
-            // The parts' sum carried on from the pressure: p + (keep - 1) * part - flux per axis.
-            const T keep = (T)c0[axis].x;
-            const T push = SCALED ? (T)c0[axis].y * scale : (T)c0[axis].y;
-            const T flux = push * (above[axis] - below[axis]);
-            total += (keep - (T)1) * part[axis] - flux;
-            part[axis] = keep * part[axis] - flux;
-            continue;
-        }
-        if (f.traj_tangent && (tangent_axes & (1u << axis))) {
-            // The step's factors along the tangent: its products with the adjoints of the new part
-            // and faces give the gradient's step (fdtd_adjoint.cuh), in double.
-            const double2 tc = g.tangent_centre[axis][at[axis]];
-            const double2 t0 = g.tangent_face[axis][at[axis]], t1 = g.tangent_face[axis][at[axis] + 1];
-            T *o = f.traj_tangent + tangent_slot;
-            tangent_slot += 3;
-            o[0] = (T)((double)part[axis] * tc.x - (double)scale * (double)(above[axis] - below[axis]) * tc.y);
-            o[1] = (T)((double)old_above[axis] * t1.x - (double)(hi[axis] - here) * t1.y);
-            o[2] = (T)((double)old_below[axis] * t0.x - (double)(here - lo[axis]) * t0.y);
-        }
-        if (f.traj_layer) {
-            T *o = f.traj_layer + (uint64_t)(6 * axis) * L + c;
-            o[0] = part[axis];
-            o[(uint64_t)1 * L] = above[axis] - below[axis];
-            o[(uint64_t)2 * L] = old_above[axis];
-            o[(uint64_t)3 * L] = hi[axis] - here;
-            o[(uint64_t)4 * L] = old_below[axis];
-            o[(uint64_t)5 * L] = here - lo[axis];
-        }
-        if (SCALED) {
-            part[axis] = (T)c0[axis].x * part[axis] - ((T)c0[axis].y * scale) * (above[axis] - below[axis]);
-        } else {
-            part[axis] = (T)c0[axis].x * part[axis] - (T)c0[axis].y * (above[axis] - below[axis]);
-        }
-        total += part[axis];
-    }
-    {
-        V2 *own = reinterpret_cast<V2 *>(f.cell_new + (uint64_t)kLayerSlots * i);
-        V2 s0, s1, s2;
-        s0.x = part[0], s0.y = part[1], s1.x = part[2], s1.y = above[0], s2.x = above[1], s2.y = above[2];
-        __stcs(own, s0), __stcs(own + 1, s1), __stcs(own + 2, s2);
+    for (int j = 1; j < 4; ++j) s.lo[0].v[j] = s.hi[0].v[j - 1];
+    s.lo[1] = load_quad(old + 4 * lanes + 4 * (uint64_t)d.y);
+    s.lo[2] = load_quad(old + 5 * lanes + 4 * (uint64_t)d.z);
+}
+
+template <bool STREAM, typename T>
+__device__ __forceinline__ void store_layer(T *now, const uint64_t lanes, const uint32_t q, const uint4 d, const LayerState<T> &s) {
+    const uint32_t mask = d.w & 15u;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        store_cells<STREAM>(now + a * lanes + 4 * (uint64_t)q, s.part[a], mask);
+        store_cells<STREAM>(now + (3 + a) * lanes + 4 * (uint64_t)q, s.hi[a], mask);
     }
     // The cell below owns the face when it is in the layer; else this cell keeps it there.
+    const uint32_t keep_x = mask & ~(d.w >> 4), keep_y = mask & ~(d.w >> 8), keep_z = mask & ~(d.w >> 12);
 #pragma unroll
-    for (int axis = 0; axis < 3; ++axis)
-        if (!(shared_below & (1u << axis))) __stcs(f.cell_new + (uint64_t)kLayerSlots * (i - strides[axis]) + 3 + axis, below[axis]);
+    for (int j = 0; j < 4; ++j)
+        if (keep_x & (1u << j)) store_once<STREAM>(now + 3 * lanes + 4 * (uint64_t)q + j - 1, s.lo[0].v[j]);
+    if (keep_y) store_cells<STREAM>(now + 4 * lanes + 4 * (uint64_t)d.y, s.lo[1], keep_y);
+    if (keep_z) store_cells<STREAM>(now + 5 * lanes + 4 * (uint64_t)d.z, s.lo[2], keep_z);
+}
+
+// A step of a quad's state (in place) and its new pressures. (Lanes outside the layer are worked out
+// too, and stored nowhere.)
+template <typename T, bool SCALED, bool COMP, bool STREAM>
+__device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, const uint32_t q, const uint4 d, LayerState<T> &s) {
+    const uint32_t mask = d.w & 15u, i = d.x;
+    const T *b = f.b;
+    const Quad<T> h = load_quad(b + i);
+    const Quad<T> ym = load_quad(b + i - g.pitch), yp = load_quad(b + i + g.pitch);
+    const Quad<T> zm = load_quad(b + i - g.plane), zp = load_quad(b + i + g.plane);
+    const T left = b[i - 1], right = b[i + 4];
+    const uint32_t z = g.by_plane(i), r = i - z * g.plane, y = g.by_pitch(r), x = r - y * g.pitch;
+    const Quad<T> sc = scales<T, SCALED>(g.lane_scale, 4 * q);
+    const bool recording = f.traj_layer || f.traj_tangent;
+    Quad<T> total{};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const uint32_t at = a == 0 ? x : (a == 1 ? y : z);
+        // (The table along x is padded to the pitch: a quad's lanes beyond the grid read it too.)
+        float4 c[5];
+#pragma unroll
+        for (int j = 0; j < (a == 0 ? 5 : 2); ++j) c[j] = __ldg(g.layer_coef[a] + at + j);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 c0 = a == 0 ? c[j] : c[0], c1 = a == 0 ? c[j + 1] : c[1];
+            const T here = h.v[j];
+            const T lo = a == 0 ? (j == 0 ? left : h.v[j - 1]) : (a == 1 ? ym.v[j] : zm.v[j]);
+            const T hi = a == 0 ? (j == 3 ? right : h.v[j + 1]) : (a == 1 ? yp.v[j] : zp.v[j]);
+            const T old_below = s.lo[a].v[j], old_above = s.hi[a].v[j], before = s.part[a].v[j];
+            const T below = (T)c0.z * old_below - (T)c0.w * (here - lo);
+            const T above = (T)c1.z * old_above - (T)c1.w * (hi - here);
+            if (recording && (mask & (1u << j))) {
+                const uint32_t cell = g.lane_cell[4 * (uint64_t)q + j];
+                const uint32_t axes = f.traj_tangent ? g.tangent_axes[cell] : 0u;
+                if (axes & (1u << a)) {
+                    // The step's factors along the tangent: its products with the adjoints of the new
+                    // part and faces give the gradient's step (fdtd_adjoint.cuh), in double.
+                    const uint32_t x0 = a == 0 ? x + j : at;
+                    const double2 tc = g.tangent_centre[a][x0];
+                    const double2 t0 = g.tangent_face[a][x0], t1 = g.tangent_face[a][x0 + 1];
+                    T *o = f.traj_tangent + g.tangent_start[cell] + 3 * __popc(axes & ((1u << a) - 1u));
+                    o[0] = (T)((double)before * tc.x - (double)sc.v[j] * (double)(above - below) * tc.y);
+                    o[1] = (T)((double)old_above * t1.x - (double)(hi - here) * t1.y);
+                    o[2] = (T)((double)old_below * t0.x - (double)(here - lo) * t0.y);
+                }
+                if (f.traj_layer) {
+                    const uint64_t L = g.layers;
+                    T *o = f.traj_layer + (uint64_t)(6 * a) * L + cell;
+                    o[0] = before;
+                    o[1 * L] = above - below;
+                    o[2 * L] = old_above;
+                    o[3 * L] = hi - here;
+                    o[4 * L] = old_below;
+                    o[5 * L] = here - lo;
+                }
+            }
+            const T push = SCALED ? (T)c0.y * sc.v[j] : (T)c0.y;
+            const T flux = push * (above - below);
+            if (COMP) {
+                // The parts' sum carried on from the pressure: p + (keep - 1) * part - flux per axis.
+                total.v[j] += ((T)c0.x - (T)1) * before - flux;
+                s.part[a].v[j] = (T)c0.x * before - flux;
+            } else {
+                s.part[a].v[j] = (T)c0.x * before - flux;
+                total.v[j] += s.part[a].v[j];
+            }
+            s.lo[a].v[j] = below, s.hi[a].v[j] = above;
+        }
+    }
     if (COMP) {
-        f.a[i] = here + total;
-        f.d[i] = total;  // (read by no update; it keeps the state's level before readable)
+        Quad<T> next;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) next.v[j] = h.v[j] + total.v[j];
+        store_cells<STREAM>(f.a + i, next, mask);
+        store_cells<STREAM>(f.d + i, total, mask);  // (read by no update; it keeps the state's level before readable)
     } else {
-        __stcs(f.a + i, total);
+        store_cells<STREAM>(f.a + i, total, mask);
     }
 }
 
+template <typename T, bool SCALED, bool COMP, bool STREAM = true>
+__device__ __forceinline__ void layer_quad(const Tables &g, const Fields<T> &f, const uint32_t q, const uint4 d) {
+    if (!(d.w & 15u)) return;  // (it only keeps a face for the quads above)
+    LayerState<T> s;
+    load_layer(f.cell_old, g.layer_lanes, q, d, s);
+    step_layer<T, SCALED, COMP, STREAM>(g, f, q, d, s);
+    store_layer<STREAM>(f.cell_new, g.layer_lanes, q, d, s);
+}
+
 // A grid of a few blocks an SM (the sweep's blocks keep their places beside it), each thread taking
-// cells c, c + the grid's threads, ...; the next cell's index is loaded while this cell's loads are
-// in flight, so that a cell costs one round trip to memory rather than two.
+// quads q, q + the grid's threads, ...; the next quad's entry is loaded while this one's loads are
+// in flight, so that a quad costs one round trip to memory rather than two.
 template <typename T, bool SCALED, bool COMP = false>
 __global__ void __launch_bounds__(kBlock) layer_kernel(const Tables g, const Fields<T> f) {
-    const uint32_t L = g.layers;
+    const uint32_t n = g.layer_quads;
     const uint32_t step = gridDim.x * kBlock;
-    uint32_t c = blockIdx.x * kBlock + threadIdx.x;
-    if (c >= L) return;
-    uint32_t next = g.layer_cells[c];
-    for (; c < L; c += step) {
-        const uint32_t i = next;
-        if (c + step < L) next = g.layer_cells[c + step];
-        layer_cell<T, SCALED, COMP>(g, f, c, i);
+    uint32_t q = blockIdx.x * kBlock + threadIdx.x;
+    if (q >= n) return;
+    uint4 next = __ldg(g.layer_quad + q);
+    for (; q < n; q += step) {
+        const uint4 entry = next;
+        if (q + step < n) next = __ldg(g.layer_quad + q + step);
+        layer_quad<T, SCALED, COMP>(g, f, q, entry);
     }
 }
 
