@@ -54,6 +54,7 @@ constexpr uint64_t kGraphSteps = 64;  // steps of fdtd_run's captured chunk (eve
 // overlapped less). Smaller grids replay the graph: below some 10M cells a step's launches and
 // event waits cost as much host time as the step takes on the device.
 constexpr uint64_t kGraphCells = 1ull << 25;
+constexpr uint64_t kGatheredSteps = 1024;  // steps the probes' cells are gathered over at most (even)
 
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
@@ -145,6 +146,10 @@ struct fdtd_solver {
     // holds the latest values between runs, as u[1] does.
     void *layer_state[2] = {nullptr, nullptr};
     uint32_t link_slots = 0;  // the most links of a special row (6 or 18 kernels)
+    // The probes' cells gathered over a piece of a run (probe_sum_kernel).
+    void *gathered = nullptr;
+    uint32_t gathered_count = 0;
+    uint64_t gathered_steps = 0;
     // Moving air (fdtd_flow.cuh): whether the grid's air moves, which form carries it, the carry's
     // cell lists, fields and stage buffers, and its launches' blocks.
     bool flowing = false, flow_round = false;
@@ -686,15 +691,27 @@ int launch_carry(fdtd_solver *s, const Fields<T> &f, cudaStream_t stream) {
     return FDTD_OK;
 }
 
-template <typename T, bool WIDE, bool SCALED, bool COMP = false>
-int launch_steps(fdtd_solver *s, const float *d_signal, uint64_t steps, double *d_out, uint64_t stride) {
+template <typename T>
+int sum_probes(fdtd_solver *s, uint64_t steps, double *d_out, uint64_t stride) {
+    const uint32_t blocks = (uint32_t)((steps * s->probes + kBlock - 1) / kBlock);
+    probe_sum_kernel<T><<<blocks, kBlock, 0, s->stream>>>(s->tables, static_cast<const T *>(s->gathered), s->gathered_count,
+                                                          (uint32_t)steps, d_out, stride);
+    CUDA_TRY(s, cudaGetLastError());
+    return FDTD_OK;
+}
+
+template <typename T, bool WIDE, bool SCALED, bool COMP>
+int launch_piece(fdtd_solver *s, const float *d_signal, uint64_t steps, double *d_out, uint64_t stride) {
     const Tables &g = s->tables;
     // The layer and special kernels loop over their cells: a few blocks an SM each (the handle's
     // layer_per_sm, special_per_sm; 0: a thread a cell), leaving the sweep's blocks their places.
     const uint64_t special_cap = s->special_per_sm ? (uint64_t)s->sms * s->special_per_sm : UINT64_MAX;
     const uint64_t layer_cap = s->layer_per_sm ? (uint64_t)s->sms * s->layer_per_sm : UINT64_MAX;
-    const uint32_t special_blocks = (uint32_t)std::min<uint64_t>((s->specials + kBlock - 1) / kBlock, special_cap);
-    const uint32_t probe_blocks = (uint32_t)((s->probes + kProbeWarps - 1) / kProbeWarps);
+    const bool probes = s->probes && s->record_probes;
+    const uint32_t gathered = probes && !s->flowing ? s->gathered_count : 0;
+    const uint32_t special_blocks = (uint32_t)std::min<uint64_t>(
+        (std::max<uint64_t>(s->specials, gathered) + kBlock - 1) / kBlock, special_cap);
+    const uint32_t probe_blocks = probes && s->flowing ? (uint32_t)((s->probes + kProbeWarps - 1) / kProbeWarps) : 0;
     const uint32_t layer_blocks = (uint32_t)std::min<uint64_t>((g.layer_quads + kBlock - 1) / kBlock, layer_cap);
     // Each step: the interior sweep on the handle's stream; beside it the matched layer on the
     // layer stream, of the highest priority (its blocks take the thread slots that the sweep's
@@ -736,6 +753,8 @@ int launch_steps(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
         f.signal = d_signal + k;
         f.out = d_out + k;
         f.out_stride = stride;
+        f.gathered = static_cast<T *>(s->gathered) + k * gathered;
+        f.gathered_count = gathered;
         if (s->record_u) {
             // The special rows' new values, level k + record_offset of the trajectory.
             f.traj_u = static_cast<T *>(s->record_u) + (k + s->record_offset) * s->specials;
@@ -754,7 +773,7 @@ int launch_steps(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
         // Moving air: the probes read the levels before the carry moves them (fdtd.hpp:833-840
         // after the record of fdtd.hpp:3525-3533); the step's updates follow the carry.
         if (s->flowing) {
-            if (probe_blocks && s->record_probes) probe_kernel<T><<<probe_blocks, kBlock, 0, s->stream>>>(g, f);
+            if (probe_blocks) probe_kernel<T><<<probe_blocks, kBlock, 0, s->stream>>>(g, f);
             launch_carry<T>(s, f, s->stream);
         }
         if (fork) {
@@ -810,8 +829,6 @@ int launch_steps(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
         }
         if (ev) CUDA_TRY(s, cudaEventRecord(ev[5], side));
         if (ev) CUDA_TRY(s, cudaEventRecord(ev[6], side));
-        // (A recomputation for the gradient records the special rows instead of the probes.)
-        if (probe_blocks && s->record_probes && !s->flowing) probe_kernel<T><<<probe_blocks, kBlock, 0, side>>>(g, f);
         if (ev) CUDA_TRY(s, cudaEventRecord(ev[7], side));
         if (fork) {
             CUDA_TRY(s, cudaEventRecord(s->joined[1], side));
@@ -824,6 +841,19 @@ int launch_steps(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
         if (layer_blocks) CUDA_TRY(s, cudaStreamWaitEvent(s->stream, s->joined[2], 0));
     }
     CUDA_TRY(s, cudaGetLastError());
+    return gathered ? sum_probes<T>(s, steps, d_out, stride) : FDTD_OK;
+}
+
+// The steps by a launch a kind of work, in pieces of at most gathered_steps steps (an even count: the
+// levels' roles return), each followed by its probes' sums.
+template <typename T, bool WIDE, bool SCALED, bool COMP>
+int launch_steps(fdtd_solver *s, const float *d_signal, uint64_t steps, double *d_out, uint64_t stride) {
+    for (uint64_t done = 0; done < steps;) {
+        const uint64_t count = std::min<uint64_t>(steps - done, s->gathered_steps);
+        const int rc = launch_piece<T, WIDE, SCALED, COMP>(s, d_signal + done, count, d_out + done, stride);
+        if (rc != FDTD_OK) return rc;
+        done += count;
+    }
     return FDTD_OK;
 }
 
@@ -1097,6 +1127,11 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
         g.link_count = u8;
         if ((rc = upload(s, direction.data(), direction.size(), &u8))) return rc;
         g.link_direction = u8;
+        std::vector<uint64_t> packed(K, 0);
+        for (uint64_t k = 0; k < K; ++k)
+            for (uint64_t l = L->link_start[k], n = 0; l < L->link_start[k + 1] && n < kPackedLinks; ++l, ++n)
+                packed[k] |= (uint64_t)L->link_direction[l] << (5 * n);
+        if ((rc = upload(s, packed.data(), K, &g.link_directions))) return rc;
         if ((rc = upload(s, weight.data(), weight.size(), &fp))) return rc;
         g.link_weight = fp;
         // Every row's links axial, in the directions' order, of the axial weight: masks.
@@ -1228,8 +1263,12 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
         const double *pd;
         if ((rc = upload(s, L->probe_weights, pc, &pd))) return rc;
         g.probe_weights = pd;
+        s->gathered_count = (uint32_t)pc;
     }
-    return FDTD_OK;
+    // The gathered pressures of a piece's steps: 32 MiB of them at most, 16 steps at least.
+    const uint64_t a_step = std::max<uint64_t>(1, s->gathered_count) * e;
+    s->gathered_steps = std::min<uint64_t>(kGatheredSteps, std::max<uint64_t>(16, (32ull << 20) / a_step)) / 2 * 2;
+    return zeros(s, a_step * s->gathered_steps, &s->gathered);
 }
 
 void release(fdtd_solver *s) {

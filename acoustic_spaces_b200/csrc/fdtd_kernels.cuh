@@ -508,6 +508,7 @@ struct Tables {
     // layout's order, and each row's count of links.
     uint32_t link_slots;
     const uint8_t *link_count, *link_direction;
+    const uint64_t *link_directions;  // each row's first twelve directions, five bits each from the lowest
     const float *link_weight, *coef_a, *coef_b, *coef_inv, *source;
     // Where every row's links are axial, in the directions' order, each of the axial weight (walls
     // on cell faces without a speed field), each row's links as a mask of the six directions
@@ -562,8 +563,10 @@ struct Fields {
     const T *cell_old;  // a step before
     T *cell_new;        // this step
     const float *signal;  // the step's drive at signal[0]
-    double *out;       // probe p's record at out[p * out_stride]
+    double *out;       // probe p's record at out[p * out_stride] (probe_kernel)
     uint64_t out_stride;
+    T *gathered;       // or the probes' cells' pressures, for probe_sum_kernel
+    uint32_t gathered_count;
     T *traj_u;         // when not null: each special row's new pressure at traj_u[k] (the gradient's
     T *traj_w;         // recomputation), and each branch state's new velocity at traj_w[j]
     // When not null (the gradient's recomputation of a grid with a matched layer): each layer
@@ -577,10 +580,14 @@ struct Fields {
 };
 
 // Special rows (fdtd.hpp:860-881), one a thread: its links, its branch states' flow, the update,
-// then the branch velocities. The links' table is slot-major, so that a warp's loads of a slot
-// are coalesced; all of a row's link loads are issued before the sum, which then adds them in
-// the layout's order. A state's term now * wb - before * wa is worked out again for the
-// velocities' update rather than kept: wa has not changed in between, so it is the same value.
+// then the branch velocities. The weights' table is slot-major, so that a warp's loads of a slot
+// are coalesced; all of a row's loads — its links' pressures and weights, its coefficients and its
+// first branch state — are issued before the sum, which then adds the links in the layout's order: a
+// row waits once for memory (its cell and its links' directions come with the row before), where
+// directions before pressures before states took three waits (the fitted rows of the 4 cm room:
+// 64.0 us with them, 74.1 at 8 blocks an SM before; see special_kernel). A state's term now * wb -
+// before * wa is worked out again for the velocities' update rather than kept: wa has not changed in
+// between, so it is the same value.
 // The links' tables are read once a step and the new pressure by no kernel of the same step, so
 // those go through the caches as streaming (evict-first) accesses, leaving L2 to the pressures
 // that the sweep and the layer share with the rows (measured: the concurrent step 2 % shorter).
@@ -598,92 +605,128 @@ __device__ __forceinline__ void store_once(V *p, V value) {
         *p = value;
 }
 
+// What a row's loads start from: its cell, its links (their count and directions, or with axial links
+// alone their mask) and its branch states.
+struct RowEntry {
+    uint32_t cell = 0, links = 0, s0 = 0, s1 = 0;
+    uint64_t directions = 0;
+};
+
+template <int SLOTS, bool STREAM>
+__device__ __forceinline__ RowEntry row_entry(const Tables &g, uint32_t k) {
+    RowEntry e;
+    e.cell = g.special[k];
+    if (SLOTS == 0) {
+        e.links = g.link_mask[k];
+    } else {
+        e.links = load_once<STREAM>(g.link_count + k);
+        e.directions = load_once<STREAM>(g.link_directions + k);
+    }
+    e.s0 = g.state_start[k], e.s1 = g.state_start[k + 1];
+    return e;
+}
+
+constexpr int kPackedLinks = 12;  // the directions a RowEntry holds
+
+// (offset: the directions' steps in the pitched grid, in shared memory: lanes index it apart.)
 template <typename T, int SLOTS, bool COMP, bool STREAM = true>
-__device__ __forceinline__ void special_row(const Tables &g, const Fields<T> &f, const uint32_t k, const uint32_t i,
-                                            const uint32_t links, const uint32_t s0, const uint32_t s1) {
-    const uint32_t K = g.specials;
+__device__ __forceinline__ void special_row(const Tables &g, const Fields<T> &f, const uint32_t k, const RowEntry &e,
+                                            const int32_t *offset) {
+    const uint32_t K = g.specials, i = e.cell;
     const T *b = f.b;
-    T sum = 0;
-    T here;
+    T value[SLOTS ? SLOTS : 6];
+    float weight[SLOTS ? SLOTS : 1];
     if constexpr (SLOTS == 0) {
         // The links as a mask of the axial directions, in their order, each of the axial weight.
-        const uint32_t mask = g.link_mask[k];
-        T value[6];
 #pragma unroll
-        for (int d = 0; d < 6; ++d) value[d] = (mask >> d) & 1u ? b[(uint32_t)((int64_t)i + g.offset[d])] : (T)0;
-        here = b[i];
-        const T w = (T)g.link_axial;
-#pragma unroll
-        for (int d = 0; d < 6; ++d)
-            if ((mask >> d) & 1u) sum += COMP ? w * (value[d] - here) : w * value[d];
+        for (int d = 0; d < 6; ++d) value[d] = (e.links >> d) & 1u ? b[i + (uint32_t)g.offset[d]] : (T)0;
     } else {
-        T value[SLOTS];
-        float weight[SLOTS];
 #pragma unroll
         for (int l = 0; l < SLOTS; ++l) {
             value[l] = (T)0;
             weight[l] = 0.0f;
-            if ((uint32_t)l < links) {
+            if ((uint32_t)l < e.links) {
                 const uint32_t at = l * K + k;
+                const uint32_t d = l < kPackedLinks ? (uint32_t)(e.directions >> (5 * l)) & 31u
+                                                    : (uint32_t)load_once<STREAM>(g.link_direction + at);
+                value[l] = b[i + (uint32_t)offset[d]];
                 weight[l] = load_once<STREAM>(g.link_weight + at);
-                value[l] = b[(uint32_t)((int64_t)i + g.offset[load_once<STREAM>(g.link_direction + at)])];
             }
         }
-        here = b[i];
+    }
+    const T here = b[i], previous = COMP ? f.d[i] : f.a[i];
+    const T ca = (T)g.coef_a[k], cb = (T)g.coef_b[k], ci = (T)g.coef_inv[k], drive = (T)g.source[k] * (T)f.signal[0];
+    T weight0 = 0, now0 = 0, before0 = 0, gain0 = 0, wb0 = 0, wa0 = 0;  // the first branch state
+    if (e.s0 < e.s1) {
+        weight0 = (T)g.state_weight[e.s0], now0 = (T)g.state_now[e.s0], before0 = (T)g.state_before[e.s0];
+        gain0 = (T)g.state_gain[e.s0], wb0 = f.wb[e.s0], wa0 = f.wa[e.s0];
+    }
+    T sum = 0;
+    if constexpr (SLOTS == 0) {
+        const T w = (T)g.link_axial;
+#pragma unroll
+        for (int d = 0; d < 6; ++d)
+            if ((e.links >> d) & 1u) sum += COMP ? w * (value[d] - here) : w * value[d];
+    } else {
 #pragma unroll
         for (int l = 0; l < SLOTS; ++l)
-            if ((uint32_t)l < links) sum += COMP ? (T)weight[l] * (value[l] - here) : (T)weight[l] * value[l];
+            if ((uint32_t)l < e.links) sum += COMP ? (T)weight[l] * (value[l] - here) : (T)weight[l] * value[l];
     }
+    const T own0 = now0 * wb0 - before0 * wa0;
     T flow = 0;
-    for (uint32_t j = s0; j < s1; ++j) {
+    if (e.s0 < e.s1) flow += weight0 * own0;
+    for (uint32_t j = e.s0 + 1; j < e.s1; ++j) {
         const T own = (T)g.state_now[j] * f.wb[j] - (T)g.state_before[j] * f.wa[j];
         flow += (T)g.state_weight[j] * own;
     }
+    T change;
     if (COMP) {
-        const T before = f.d[i];
-        const T step = (sum + (T)g.coef_b[k] * before - flow + (T)g.source[k] * (T)f.signal[0]) * (T)g.coef_inv[k] +
-                       (T)g.row_residual[k] * here;
+        const T step = (sum + cb * previous - flow + drive) * ci + (T)g.row_residual[k] * here;
         f.a[i] = here + step;
         f.d[i] = step;
-        for (uint32_t j = s0; j < s1; ++j) {
-            const T own = (T)g.state_now[j] * f.wb[j] - (T)g.state_before[j] * f.wa[j];
-            f.wa[j] = f.wa[j] + ((step + before) * (T)g.state_gain[j] + own);
-        }
-        return;
+        change = step + previous;
+    } else {
+        const T next = (ca * here + sum - cb * previous - flow + drive) * ci;
+        store_once<STREAM>(f.a + i, next);
+        if (f.traj_u) f.traj_u[k] = next;
+        change = next - previous;
     }
-    const T previous = f.a[i];
-    const T next = ((T)g.coef_a[k] * here + sum - (T)g.coef_b[k] * previous - flow +
-                    (T)g.source[k] * (T)f.signal[0]) * (T)g.coef_inv[k];
-    store_once<STREAM>(f.a + i, next);
-    if (f.traj_u) f.traj_u[k] = next;
-    for (uint32_t j = s0; j < s1; ++j) {
+    if (e.s0 < e.s1) {
+        const T w = wa0 + (change * gain0 + own0);
+        f.wa[e.s0] = w;
+        if (!COMP && f.traj_w) f.traj_w[e.s0] = w;
+    }
+    for (uint32_t j = e.s0 + 1; j < e.s1; ++j) {
         const T own = (T)g.state_now[j] * f.wb[j] - (T)g.state_before[j] * f.wa[j];
-        const T w = f.wa[j] + ((next - previous) * (T)g.state_gain[j] + own);
+        const T w = f.wa[j] + (change * (T)g.state_gain[j] + own);
         f.wa[j] = w;
-        if (f.traj_w) f.traj_w[j] = w;
+        if (!COMP && f.traj_w) f.traj_w[j] = w;
     }
 }
 
-// Rows k, k + the grid's threads, ... a thread, the next row's cell index, link count and branch
-// states' bounds loaded while this row's loads are in flight, so that a row's link loads wait on
-// no load of its own (measured: the kernel 10 % shorter on the fitted rows).
+// The probes' cells' pressures before the step, in their order, by the grid's threads.
+template <typename T>
+__device__ __forceinline__ void gather_probes(const Tables &g, const Fields<T> &f, uint32_t first, uint32_t step) {
+    for (uint32_t e = first; e < f.gathered_count; e += step) f.gathered[e] = f.b[g.probe_cells[e]];
+}
+
+// Rows k, k + the grid's threads, ... a thread, the next row's entry loaded while this row's loads are
+// in flight; then the probes' cells.
 template <typename T, int SLOTS, bool COMP = false>
 __global__ void __launch_bounds__(kBlock) special_kernel(const Tables g, const Fields<T> f) {
+    __shared__ int32_t offset[18];
+    if (threadIdx.x < 18) offset[threadIdx.x] = g.offset[threadIdx.x];
+    __syncthreads();
     const uint32_t K = g.specials;
     const uint32_t step = gridDim.x * kBlock;
     uint32_t k = blockIdx.x * kBlock + threadIdx.x;
+    gather_probes<T>(g, f, k, step);
     if (k >= K) return;
-    uint32_t next = g.special[k];
-    uint32_t next_links = SLOTS ? (uint32_t)__ldcs(g.link_count + k) : 0u;
-    uint32_t next_s0 = g.state_start[k], next_s1 = g.state_start[k + 1];
+    RowEntry next = row_entry<SLOTS, true>(g, k);
     for (; k < K; k += step) {
-        const uint32_t i = next, links = next_links, s0 = next_s0, s1 = next_s1;
-        if (k + step < K) {
-            next = g.special[k + step];
-            if (SLOTS) next_links = __ldcs(g.link_count + k + step);
-            next_s0 = g.state_start[k + step], next_s1 = g.state_start[k + step + 1];
-        }
-        special_row<T, SLOTS, COMP>(g, f, k, i, links, s0, s1);
+        const RowEntry e = next;
+        if (k + step < K) next = row_entry<SLOTS, true>(g, k + step);
+        special_row<T, SLOTS, COMP>(g, f, k, e, offset);
     }
 }
 
@@ -786,7 +829,8 @@ __device__ __forceinline__ void store_layer(T *now, const uint64_t lanes, const 
 // A step of a quad's state (in place) and its new pressures. (Lanes outside the layer are worked out
 // too, and stored nowhere.)
 template <typename T, bool SCALED, bool COMP, bool STREAM>
-__device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, const uint32_t q, const uint4 d, LayerState<T> &s) {
+__device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, const float4 *const (&coef)[3], const uint32_t q,
+                                           const uint4 d, LayerState<T> &s) {
     const uint32_t mask = d.w & 15u, i = d.x;
     const T *b = f.b;
     const Quad<T> h = load_quad(b + i);
@@ -803,7 +847,7 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
         // (The table along x is padded to the pitch: a quad's lanes beyond the grid read it too.)
         float4 c[5];
 #pragma unroll
-        for (int j = 0; j < (a == 0 ? 5 : 2); ++j) c[j] = __ldg(g.layer_coef[a] + at + j);
+        for (int j = 0; j < (a == 0 ? 5 : 2); ++j) c[j] = coef[a][at + j];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const float4 c0 = a == 0 ? c[j] : c[0], c1 = a == 0 ? c[j + 1] : c[1];
@@ -867,7 +911,7 @@ __device__ __forceinline__ void layer_quad(const Tables &g, const Fields<T> &f, 
     if (!(d.w & 15u)) return;  // (it only keeps a face for the quads above)
     LayerState<T> s;
     load_layer(f.cell_old, g.layer_lanes, q, d, s);
-    step_layer<T, SCALED, COMP, STREAM>(g, f, q, d, s);
+    step_layer<T, SCALED, COMP, STREAM>(g, f, g.layer_coef, q, d, s);
     store_layer<STREAM>(f.cell_new, g.layer_lanes, q, d, s);
 }
 
@@ -891,7 +935,7 @@ __global__ void __launch_bounds__(kBlock) layer_kernel(const Tables g, const Fie
 // Probe p's pressure before the step (fdtd.hpp:3525-3533): its cells' weighted sum in double, in
 // the layout's order. A warp per probe: the lanes load the cells and form the products (each
 // product is the reference's own), then lane 0 adds them up in the layout's order, so that the
-// sum rounds as the reference's sequential one.
+// sum rounds as the reference's sequential one. (Moving air, whose carry follows the record.)
 constexpr int kProbeWarps = kBlock / 32;
 
 template <typename T>
@@ -911,6 +955,21 @@ __global__ void __launch_bounds__(kBlock) probe_kernel(const Tables g, const Fie
         }
     }
     if (lane == 0) f.out[(uint64_t)p * f.out_stride] = value;
+}
+
+// The same records from the pressures that the steps gathered, a thread a probe and step: a sum's 64
+// dependent additions take half a microsecond, and one such launch a step took 9.6 us alone at the
+// end of the special rows (16 probes); of many steps at once they take as long together.
+template <typename T>
+__global__ void __launch_bounds__(kBlock) probe_sum_kernel(const Tables g, const T *gathered, uint32_t count,
+                                                           uint32_t steps, double *out, uint64_t stride) {
+    const uint64_t e = (uint64_t)blockIdx.x * kBlock + threadIdx.x;
+    if (e >= (uint64_t)steps * g.probes) return;
+    const uint32_t p = (uint32_t)(e / steps), k = (uint32_t)(e - (uint64_t)p * steps);
+    const T *read = gathered + (uint64_t)k * count;
+    double value = 0.0;
+    for (uint32_t c = g.probe_start[p], end = g.probe_start[p + 1]; c < end; ++c) value += g.probe_weights[c] * (double)read[c];
+    out[(uint64_t)p * stride + k] = value;
 }
 
 }  // namespace fdtd
