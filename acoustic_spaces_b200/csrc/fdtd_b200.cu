@@ -27,6 +27,7 @@
 #include "fdtd_b200.h"
 #include "fdtd_flow.cuh"
 #include "fdtd_kernels.cuh"
+#include "fdtd_resident.cuh"
 
 using namespace fdtd;
 
@@ -54,6 +55,7 @@ constexpr uint64_t kGraphSteps = 64;  // steps of fdtd_run's captured chunk (eve
 // overlapped less). Smaller grids replay the graph: below some 10M cells a step's launches and
 // event waits cost as much host time as the step takes on the device.
 constexpr uint64_t kGraphCells = 1ull << 25;
+constexpr uint32_t kResidentSmem = 216 * 1024;  // shared memory a block of the resident stepper takes at most
 constexpr uint64_t kGatheredSteps = 1024;  // steps the probes' cells are gathered over at most (even)
 
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -146,7 +148,17 @@ struct fdtd_solver {
     // holds the latest values between runs, as u[1] does.
     void *layer_state[2] = {nullptr, nullptr};
     uint32_t link_slots = 0;  // the most links of a special row (6 or 18 kernels)
-    // The probes' cells gathered over a piece of a run (probe_sum_kernel).
+    // The resident stepper (fdtd_resident.cuh): whether the grid takes it, its interior's columns, the
+    // launch's blocks (one cluster of them, or as many as the GPU holds at once), the barriers'
+    // count and the probes' cells gathered over a launch's steps.
+    bool resident = false, resident_clustered = false;
+    const uint2 *columns = nullptr;
+    uint32_t column_count = 0, resident_blocks = 0, resident_smem = 0;
+    bool resident_staged = false;
+    uint32_t resident_keep_layer = 0, resident_rows_at = 0, resident_layer_at = 0;
+    const uint32_t *link_start = nullptr;
+    const uint2 *row_links = nullptr;
+    unsigned int *arrived = nullptr;
     void *gathered = nullptr;
     uint32_t gathered_count = 0;
     uint64_t gathered_steps = 0;
@@ -160,8 +172,9 @@ struct fdtd_solver {
     // previous-pressure tile, the cell types and the scales.
     CUtensorMap map_b[2], map_a[2], map_t, map_s;
     CUtensorMap map_d;  // FDTD_FP32_COMPENSATED: the increments, in the previous pressure's place
-    // fdtd_run's chunks: the drive and the records of kGraphSteps steps on the device, and the
+    // fdtd_run's chunks: the drive and the records of chunk_steps steps on the device, and the
     // graph of a chunk's launches for each of the levels' two roles (captured on first use).
+    uint64_t chunk_steps = kGraphSteps;
     float *d_sig = nullptr;
     double *d_rec = nullptr;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -857,9 +870,205 @@ int launch_steps(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
     return FDTD_OK;
 }
 
+// The steps by the resident stepper: pieces of at most gathered_steps steps a launch, each followed by
+// its probes' sums.
+template <typename T, bool WIDE, bool SCALED, bool COMP, bool LAYER>
+int launch_resident(fdtd_solver *s, const float *d_signal, uint64_t steps, double *d_out, uint64_t stride) {
+    const bool probes = s->probes && s->record_probes;
+    for (uint64_t done = 0; done < steps;) {
+        const uint64_t count = std::min<uint64_t>(steps - done, s->gathered_steps);
+        const int cur = done & 1 ? 0 : 1;
+        ResidentArgs<T> a{};
+        a.g = s->tables;
+        for (int k = 0; k < 2; ++k) {
+            const int from = k ? cur : 1 - cur;
+            a.u[k] = static_cast<T *>(s->u[from]), a.w[k] = static_cast<T *>(s->w[from]);
+            a.layer[k] = static_cast<T *>(s->layer_state[from]);
+        }
+        a.d = static_cast<T *>(s->increment);
+        a.scale = s->scale_device;
+        a.columns = s->columns, a.column_count = s->column_count;
+        a.axial = s->bulk.axial, a.diagonal = s->bulk.diagonal, a.centre = s->bulk.centre, a.total = s->bulk.total;
+        a.residual = s->bulk.residual;
+        a.signal = d_signal + done;
+        a.link_start = s->link_start, a.links = s->row_links, a.staged = s->resident_staged ? 1 : 0;
+        a.keep_layer = s->resident_keep_layer, a.rows_at = s->resident_rows_at, a.layer_at = s->resident_layer_at;
+        a.coefs[0] = (uint32_t)s->pitch + 2, a.coefs[1] = (uint32_t)s->ny + 1, a.coefs[2] = (uint32_t)s->nz + 1;
+        a.gathered = static_cast<T *>(s->gathered), a.gathered_count = probes ? s->gathered_count : 0;
+        if (s->record_u) {
+            a.traj_u = static_cast<T *>(s->record_u) + (done + s->record_offset) * s->specials;
+            a.traj_w = static_cast<T *>(s->record_w) + (done + s->record_offset) * s->states;
+        }
+        if (s->record_layer) a.traj_layer = static_cast<T *>(s->record_layer) + done * kLayerFactors * s->layers;
+        if (s->record_tangent) a.traj_tangent = static_cast<T *>(s->record_tangent) + done * s->tangent_factors;
+        a.states = (uint32_t)s->states, a.tangent_factors = (uint32_t)s->tangent_factors;
+        a.steps = (uint32_t)count;
+        a.clustered = s->resident_clustered ? 1 : 0;
+        a.arrived = s->arrived, a.error = s->d_error;
+        cudaLaunchConfig_t config{};
+        config.gridDim = dim3(s->resident_blocks);
+        config.blockDim = dim3(kResidentThreads<T, WIDE, LAYER>);
+        config.dynamicSmemBytes = s->resident_smem;
+        config.stream = s->stream;
+        cudaLaunchAttribute attr{};
+        if (s->resident_clustered) {
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = s->resident_blocks, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        } else {
+            // The blocks wait for one another: all of them resident at once, or the launch fails.
+            attr.id = cudaLaunchAttributeCooperative;
+            attr.val.cooperative = 1;
+            CUDA_TRY(s, cudaMemsetAsync(s->arrived, 0, sizeof(unsigned int), s->stream));
+        }
+        config.attrs = &attr;
+        config.numAttrs = 1;
+        CUDA_TRY(s, cudaLaunchKernelEx(&config, resident_kernel<T, WIDE, SCALED, COMP, LAYER>, a));
+        if (probes && s->gathered_count) {
+            const int rc = sum_probes<T>(s, count, d_out + done, stride);
+            if (rc != FDTD_OK) return rc;
+        }
+        done += count;
+    }
+    return FDTD_OK;
+}
+
 template <typename T, bool W, bool S, bool C>
 int dispatch_run(fdtd_solver *s, const float *d_signal, uint64_t steps, double *d_out, uint64_t stride) {
+    if (s->resident && !s->timing)
+        return s->layers ? launch_resident<T, W, S, C, !W>(s, d_signal, steps, d_out, stride)
+                         : launch_resident<T, W, S, C, false>(s, d_signal, steps, d_out, stride);
     return launch_steps<T, W, S, C>(s, d_signal, steps, d_out, stride);
+}
+
+// The columns of quads of the interior, `planes` planes at most each: every run of planes that
+// holds interior cells, from its first, so that a column's first plane holds one.
+void interior_columns(const fdtd_solver *s, uint64_t planes, std::vector<uint2> &columns) {
+    columns.clear();
+    const BulkArgs &bk = s->bulk;
+    if (s->host_types.empty()) return;
+    const uint64_t quads = s->pitch / 4, plane = s->pitch * s->ny;
+    std::vector<uint32_t> masks(quads);
+    for (uint64_t z0 = bk.z0; z0 < bk.z1; z0 += planes)
+        for (uint64_t y = bk.y0; y < bk.y1; ++y) {
+            std::fill(masks.begin(), masks.end(), 0u);
+            for (uint64_t z = z0, end = std::min<uint64_t>(z0 + planes, bk.z1); z < end; ++z) {
+                const uint8_t *row = &s->host_types[plane * z + s->pitch * y];
+                for (uint64_t q = 0; q < quads; ++q) {
+                    uint32_t four;
+                    std::memcpy(&four, row + 4 * q, 4);
+                    if (!four) continue;
+                    uint32_t mask = 0;
+                    for (int j = 0; j < 4; ++j) mask |= (((four >> (8 * j)) & 255u) == kInterior ? 1u : 0u) << j;
+                    masks[q] |= mask << (4 * (z - z0));
+                }
+            }
+            for (uint64_t q = 0; q < quads; ++q) {
+                if (!masks[q]) continue;
+                const int skip = __builtin_ctz(masks[q]) / 4;
+                columns.push_back(make_uint2((uint32_t)(plane * (z0 + skip) + s->pitch * y + 4 * q), masks[q] >> (4 * skip)));
+            }
+        }
+}
+
+// Whether the grid takes the resident stepper: the bytes that its steps touch, against a limit.
+// Below it they stay in L2 and a step costs its barrier, not its launches; beyond it the launched
+// steps' pipelined sweep keeps more of the DRAM's bandwidth. Measured, us a step, launched and
+// resident: FP32 boxes of 6.3M cells (50 MB) 20.5 and 16.1-18.2, 11.5M (92 MB) 39-49 and 34.6-36.4, 16M (128
+// MB) 50.3 and 49.0, 21M 62.8 and 76; compensated 6.3M (75 MB) 25.7 and 20.5, 11.5M (138 MB) 48 and 53-58; with a
+// matched layer FP32 3M (0.9M layer cells, 74 MB) 28.7 and 25.6, 5.9M (131 MB) 39 and 56; the wide
+// stencil 9.7M (78 MB) 73.6 and 69.5. In double the launched sweep is the slower one and a plain box
+// still gains at 184 MB (65.8 and 59.8; at 255 MB 85.9 and 90.4), the wide stencil not beyond 61 MB (51.4
+// and 51.5 there).
+bool takes_resident(const fdtd_solver *s, const fdtd_layout *L) {
+    if (L->flow_count) return false;
+    const uint64_t e = s->precision == FDTD_FP64 ? 8 : 4, MB = 1000 * 1000;
+    const uint64_t a_cell = 2 * e + (s->precision == FDTD_FP32_COMPENSATED ? e : 0) + (s->scaled ? 4 : 0);
+    const uint64_t touched = a_cell * s->n_device + 2 * kLayerSlots * e * L->layer_count;
+    if (e == 4) return touched <= 100 * MB;
+    return touched <= (s->wide ? 50 * MB : (L->layer_count ? 80 * MB : 190 * MB));
+}
+
+// The resident stepper's launch and lists for the grid, once takes_resident has said yes.
+template <typename T, bool WIDE, bool SCALED, bool COMP, bool LAYER>
+int set_up_resident(fdtd_solver *s, const std::vector<uint32_t> &link_start, const std::vector<uint32_t> &state_start) {
+    s->resident = false;
+    if (LAYER && 16 * (s->pitch + s->ny + s->nz + 4) > kResidentSmem) return FDTD_OK;  // (a grid of lines)
+    auto kernel = resident_kernel<T, WIDE, SCALED, COMP, LAYER>;
+    const int threads = kResidentThreads<T, WIDE, LAYER>;
+    auto tasks = [](uint64_t n) { return (n + 31) / 32; };
+    const uint64_t other = tasks(s->specials) + tasks(s->tables.layer_quads) + tasks(s->gathered_count);
+    // Planes a column: as few as leave every warp one task (a step is then one chain of loads);
+    // where the tasks are more than the warps, the choice of the fewest planes in turn a warp, two
+    // planes counted for a column's first loads.
+    const uint64_t warps = (uint64_t)s->sms * (threads / 32);
+    std::vector<uint2> columns;
+    interior_columns(s, 1, columns);
+    uint64_t quads = columns.size(), best = 1;
+    double least = 1e300;
+    for (uint64_t planes = 1; planes <= kColumnPlanes; ++planes) {
+        const uint64_t rounds = (other + tasks((quads + planes - 1) / planes) + warps - 1) / warps;
+        const double cost = (double)rounds * ((double)planes + 2.0);
+        if (cost < least) least = cost, best = planes;
+    }
+    if (best > 1) interior_columns(s, best, columns);
+    int rc;
+    if ((rc = upload(s, columns.data(), columns.size(), &s->columns))) return rc;
+    s->column_count = (uint32_t)columns.size();
+    const uint64_t all = other + tasks(columns.size());
+    // Blocks: one a multiprocessor, or a cluster's where its warps take the tasks a few each: its
+    // barrier is faster than one over the whole GPU.
+    // The shared memory of a block's rows, if the largest block's fits.
+    auto stage = [&](uint32_t blocks) {
+        uint32_t most = 0;
+        for (uint32_t k = 0; k < blocks; ++k) {
+            const uint32_t r0 = std::min<uint32_t>(share_of(s->tables.specials, k, blocks) * 32, s->tables.specials);
+            const uint32_t r1 = std::min<uint32_t>(share_of(s->tables.specials, k + 1, blocks) * 32, s->tables.specials);
+            const uint32_t links = s->tables.link_mask ? 0 : link_start[r1] - link_start[r0];
+            most = std::max(most, RowStage<T>::bytes(r1 - r0, links, state_start[r1] - state_start[r0]));
+        }
+        // The layer's coefficients first, then the rows, then the state of as many of the layer's tasks
+        // as fit beside them (nine quads a quad).
+        const uint32_t coefs = LAYER ? 16 * (uint32_t)(s->pitch + 2 + s->ny + 1 + s->nz + 1) : 0;
+        s->resident_staged = coefs + most <= kResidentSmem;
+        s->resident_rows_at = (coefs + 127u) / 128u * 128u;
+        s->resident_layer_at = s->resident_rows_at + (s->resident_staged ? (most + 127u) / 128u * 128u : 0);
+        const uint32_t a_task = 9 * 128 * sizeof(T), left = kResidentSmem - std::min(kResidentSmem, s->resident_layer_at);
+        const uint64_t a_block = (tasks(s->tables.layer_quads) + blocks - 1) / blocks;
+        s->resident_keep_layer = (uint32_t)std::min<uint64_t>(a_block, left / a_task);
+        s->resident_smem = s->resident_layer_at + s->resident_keep_layer * a_task;
+    };
+    CUDA_TRY(s, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResidentSmem));
+    s->resident_blocks = (uint32_t)s->sms, s->resident_clustered = false;
+    stage(s->resident_blocks);
+    if (2 * all <= 16 * (uint64_t)(threads / 32)) {
+        uint32_t blocks = 16;
+        CUDA_TRY(s, cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        for (; blocks; blocks = blocks == 16 ? 8 : 0) {
+            stage(blocks);
+            cudaLaunchConfig_t config{};
+            config.gridDim = dim3(blocks), config.blockDim = dim3(threads), config.dynamicSmemBytes = s->resident_smem;
+            cudaLaunchAttribute attr{};
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = blocks, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            config.attrs = &attr, config.numAttrs = 1;
+            int clusters = 0;
+            CUDA_TRY(s, cudaOccupancyMaxActiveClusters(&clusters, kernel, &config));
+            if (clusters < 1) continue;
+            s->resident_blocks = blocks, s->resident_clustered = true;
+            break;
+        }
+        if (!s->resident_clustered) stage(s->resident_blocks);
+    }
+    if (!s->resident_clustered) {
+        int per_sm = 0;
+        CUDA_TRY(s, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, s->resident_smem));
+        if (per_sm < 1) return FDTD_OK;
+    }
+    void *p;
+    if ((rc = zeros(s, sizeof(unsigned int), &p))) return rc;
+    s->arrived = static_cast<unsigned int *>(p);
+    s->resident = true;
+    return FDTD_OK;
 }
 
 // The instantiation for the grid: precision (and compensated single), stencil, speed field.
@@ -885,6 +1094,13 @@ int dispatch(fdtd_solver *s, const float *d_signal, uint64_t steps, double *d_ou
 
 int set_up(fdtd_solver *s) {
 #define SET_CALL(T, W, S, C) set_up_kernels<T, W, S, C>(s)
+    FDTD_BY_KIND(SET_CALL);
+#undef SET_CALL
+}
+
+int set_up_resident_kind(fdtd_solver *s, const std::vector<uint32_t> &link_start, const std::vector<uint32_t> &state_start) {
+#define SET_CALL(T, W, S, C) \
+    (s->layers ? set_up_resident<T, W, S, C, !W>(s, link_start, state_start) : set_up_resident<T, W, S, C, false>(s, link_start, state_start))
     FDTD_BY_KIND(SET_CALL);
 #undef SET_CALL
 }
@@ -923,7 +1139,7 @@ int capture(fdtd_solver *s, cudaGraphExec_t *out) {
     const bool timing = s->timing;
     s->timing = false;  // no timing events inside a graph
     CUDA_TRY(s, cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    const int rc = dispatch(s, s->d_sig, kGraphSteps, s->d_rec, kGraphSteps);
+    const int rc = dispatch(s, s->d_sig, kGraphSteps, s->d_rec, s->chunk_steps);
     s->timing = timing;
     cudaGraph_t graph = nullptr;
     const cudaError_t e = cudaStreamEndCapture(s->stream, &graph);
@@ -1054,9 +1270,14 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
     if ((rc = zeros(s, sizeof(unsigned int), &flag))) return rc;
     s->d_error = static_cast<unsigned int *>(flag);
     void *chunk;
-    if ((rc = zeros(s, sizeof(float) * kGraphSteps, &chunk))) return rc;
+    // (The resident stepper's chunks are longer; of many probes, 8 MiB of records at most.)
+    const uint64_t P1 = std::max<uint64_t>(1, L->probe_count);
+    const bool resident = takes_resident(s, L);
+    if (resident)
+        s->chunk_steps = std::min<uint64_t>(kGatheredSteps, std::max<uint64_t>(kGraphSteps, (8ull << 20) / (8 * P1)));
+    if ((rc = zeros(s, sizeof(float) * s->chunk_steps, &chunk))) return rc;
     s->d_sig = static_cast<float *>(chunk);
-    if ((rc = zeros(s, sizeof(double) * kGraphSteps * std::max<uint64_t>(1, L->probe_count), &chunk))) return rc;
+    if ((rc = zeros(s, sizeof(double) * s->chunk_steps * P1, &chunk))) return rc;
     s->d_rec = static_cast<double *>(chunk);
     if (L->flow_count && (rc = set_up_flow(s, L))) return rc;
 
@@ -1096,8 +1317,9 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
     g.specials = (uint32_t)K;
     const float *fp;
     const uint8_t *u8;
+    std::vector<uint32_t> link_start, state_start(K + 1);
     {
-        std::vector<uint32_t> special(K), state_start(K + 1);
+        std::vector<uint32_t> special(K);
         uint64_t slots = 0;
         for (uint64_t k = 0; k < K; ++k) {
             special[k] = pitched(s, (uint64_t)L->special[k]);
@@ -1151,6 +1373,19 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
         if (axial_rows) {
             if ((rc = upload(s, mask.data(), K, &u8))) return rc;
             g.link_mask = u8;
+        }
+        if (!axial_rows && resident) {
+            // The resident stepper's links, row by row.
+            std::vector<uint2> links(L->link_count);
+            for (uint64_t l = 0; l < L->link_count; ++l) {
+                uint32_t weight_bits;
+                std::memcpy(&weight_bits, &L->link_weight[l], 4);
+                links[l] = make_uint2(weight_bits, (uint32_t)g.offset[L->link_direction[l]]);
+            }
+            link_start.resize(K + 1);
+            for (uint64_t k = 0; k <= K; ++k) link_start[k] = (uint32_t)L->link_start[k];
+            if ((rc = upload(s, links.data(), links.size(), &s->row_links))) return rc;
+            if ((rc = upload(s, link_start.data(), link_start.size(), &s->link_start))) return rc;
         }
     }
     if ((rc = upload(s, L->coef_a, K, &fp))) return rc;
@@ -1268,7 +1503,8 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
     // The gathered pressures of a piece's steps: 32 MiB of them at most, 16 steps at least.
     const uint64_t a_step = std::max<uint64_t>(1, s->gathered_count) * e;
     s->gathered_steps = std::min<uint64_t>(kGatheredSteps, std::max<uint64_t>(16, (32ull << 20) / a_step)) / 2 * 2;
-    return zeros(s, a_step * s->gathered_steps, &s->gathered);
+    if ((rc = zeros(s, a_step * s->gathered_steps, &s->gathered))) return rc;
+    return resident ? set_up_resident_kind(s, link_start, state_start) : FDTD_OK;
 }
 
 void release(fdtd_solver *s) {
@@ -1974,7 +2210,8 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
         s->graph_segment = segment;
     }
     auto run = [&](int which, int key, auto &&body, uint64_t count) -> int {
-        if (!graphs || count != segment || segments == 1) return body(count);
+        // (The resident stepper's recomputation is a launch or two: nothing to capture.)
+        if (!graphs || count != segment || segments == 1 || (which == 0 && s->resident && !s->timing)) return body(count);
         cudaGraphExec_t &exec = s->grad_graph[which][key];
         if (!exec) {
             const bool timing = s->timing;
@@ -2338,9 +2575,10 @@ int fdtd_run(fdtd_solver *s, const float *signal, uint64_t steps, double *out) {
     if (!signal || (s->probes && !out)) return fail(s, FDTD_EINVAL, "no signal or output buffer");
     DeviceGuard guard(s->device);
     // Pinned host staging for a piece of the run (the drive and the probes' records), grown on
-    // demand; the device side is the handle's chunk buffers, kGraphSteps steps at a time.
+    // demand; the device side is the handle's chunk buffers, chunk_steps steps at a time.
     const uint64_t P = std::max<uint64_t>(1, s->probes);
-    const uint64_t piece = std::min<uint64_t>(steps, std::max<uint64_t>(kGraphSteps, (64ull << 20) / (8 * P)));
+    const bool resident = s->resident && !s->timing;  // (its chunks are no captured graphs)
+    const uint64_t piece = std::min<uint64_t>(steps, std::max<uint64_t>(s->chunk_steps, (64ull << 20) / (8 * P)));
     if (s->stage_steps < piece) {
         if (s->stage_signal) cudaFreeHost(s->stage_signal);
         if (s->stage_out) cudaFreeHost(s->stage_out);
@@ -2394,7 +2632,7 @@ int fdtd_run(fdtd_solver *s, const float *signal, uint64_t steps, double *out) {
             if ((r = zeros(s, e * S * (steps + 2), &s->tape_w)) != FDTD_OK) return r;
             s->tape_levels = steps + 2;
         }
-        if (!s->stage_u) {
+        if (!s->stage_u && !resident) {
             if ((r = zeros(s, e * K * kGraphSteps, &s->stage_u)) != FDTD_OK) return r;
             if ((r = zeros(s, e * S * kGraphSteps, &s->stage_w)) != FDTD_OK) return r;
         }
@@ -2408,7 +2646,7 @@ int fdtd_run(fdtd_solver *s, const float *signal, uint64_t steps, double *out) {
             if ((r = zeros(s, e * s->tangent_factors * steps, &s->tape_t)) != FDTD_OK) return r;
             s->tape_t_steps = steps;
         }
-        if (keep_tangent && !s->stage_t && (r = zeros(s, e * s->tangent_factors * kGraphSteps, &s->stage_t)) != FDTD_OK)
+        if (keep_tangent && !resident && !s->stage_t && (r = zeros(s, e * s->tangent_factors * kGraphSteps, &s->stage_t)) != FDTD_OK)
             return r;
         // Levels 0 and 1: the state at rest.
         CUDA_TRY(s, cudaMemsetAsync(s->tape_u, 0, e * K * 2, s->stream));
@@ -2436,26 +2674,29 @@ int fdtd_run(fdtd_solver *s, const float *signal, uint64_t steps, double *out) {
         const uint64_t count = std::min(piece, steps - begin);
         std::memcpy(s->stage_signal, signal + begin, count * sizeof(float));
         for (uint64_t done = 0; done < count && rc == FDTD_OK;) {
-            uint64_t chunk = std::min<uint64_t>(kGraphSteps, count - done);
+            uint64_t chunk = std::min<uint64_t>(resident ? s->chunk_steps : kGraphSteps, count - done);
             const uint64_t at = begin + done;  // steps of this run done before the chunk
             if (taping) chunk = std::min(chunk, (at / tape_segment + 1) * tape_segment - at);
             CUDA_TRY(s, cudaMemcpyAsync(s->d_sig, s->stage_signal + done, chunk * sizeof(float), cudaMemcpyHostToDevice,
                                         s->stream));
-            const bool graphed = chunk == kGraphSteps && s->n_device < kGraphCells;
+            const bool graphed = chunk == kGraphSteps && s->n_device < kGraphCells && !resident;
             // (The tangent's factors: straight onto the tape, or a captured chunk's into staging.)
             if (keep_tangent)
                 s->record_tangent = graphed ? s->stage_t : static_cast<char *>(s->tape_t) + e * s->tangent_factors * at;
+            if (keep_traj && resident)  // (its launches are given their places on the tape)
+                s->record_u = static_cast<char *>(s->tape_u) + e * K * (at + 2),
+                s->record_w = static_cast<char *>(s->tape_w) + e * S * (at + 2);
             if (graphed) {
                 // A whole chunk: the captured graph of its steps for the levels' present roles
                 // (with the trajectory's recording, a graph of its own).
                 cudaGraphExec_t &graph = keep_traj ? s->tape_graph[s->flipped ? 1 : 0] : s->graph[s->flipped ? 1 : 0];
                 if (!graph && (rc = capture(s, &graph)) != FDTD_OK) break;
                 CUDA_TRY(s, cudaGraphLaunch(graph, s->stream));
-            } else if ((rc = dispatch(s, s->d_sig, chunk, s->d_rec, kGraphSteps)) != FDTD_OK) {
+            } else if ((rc = dispatch(s, s->d_sig, chunk, s->d_rec, s->chunk_steps)) != FDTD_OK) {
                 break;
             }
             settle(s, chunk);
-            if (keep_traj) {
+            if (keep_traj && !resident) {
                 // The chunk's levels at + 2 .. at + chunk + 1 onto the tape.
                 CUDA_TRY(s, cudaMemcpyAsync(static_cast<char *>(s->tape_u) + e * K * (at + 2), s->stage_u, e * K * chunk,
                                             cudaMemcpyDeviceToDevice, s->stream));
@@ -2472,7 +2713,7 @@ int fdtd_run(fdtd_solver *s, const float *signal, uint64_t steps, double *out) {
             }
             if (s->probes) {
                 CUDA_TRY(s, cudaMemcpy2DAsync(s->stage_out + done, count * sizeof(double), s->d_rec,
-                                              kGraphSteps * sizeof(double), chunk * sizeof(double), s->probes,
+                                              s->chunk_steps * sizeof(double), chunk * sizeof(double), s->probes,
                                               cudaMemcpyDeviceToHost, s->stream));
             }
             done += chunk;
@@ -2719,6 +2960,7 @@ int fdtd_set_launch(fdtd_solver *s, int layer_per_sm, int special_per_sm) {
     DeviceGuard guard(s->device);
     for (cudaStream_t stream : {s->stream, s->side, s->layer_stream}) CUDA_TRY(s, cudaStreamSynchronize(stream));
     s->layer_per_sm = layer_per_sm, s->special_per_sm = special_per_sm;
+    s->resident = false;  // (the caller chooses the launches' shapes: the steps are launched)
     // The captured chunks and the gradient's graphs hold the old launch shapes.
     Kept{s}.drop_graphs();
     for (cudaGraphExec_t &g : s->graph)
@@ -2738,6 +2980,7 @@ int fdtd_set_tiles(fdtd_solver *s, int shape, uint64_t planes) {
     DeviceGuard guard(s->device);
     for (cudaStream_t stream : {s->stream, s->side, s->layer_stream}) CUDA_TRY(s, cudaStreamSynchronize(stream));
     Kept{s}.drop_graphs();
+    s->resident = false;
     return use_shape(s, shape, planes);
 }
 
@@ -2773,6 +3016,7 @@ int fdtd_set_streams(fdtd_solver *s, int concurrent) {
     for (cudaStream_t stream : {s->stream, s->side, s->layer_stream}) CUDA_TRY(s, cudaStreamSynchronize(stream));
     if (concurrent < 0 || concurrent > 5) return fail(s, FDTD_EINVAL, "the streams' arrangement is 0 to 5");
     s->concurrent = concurrent;
+    s->resident = false;
     // The captured chunks and the gradient's graphs hold the old streams' order.
     Kept{s}.drop_graphs();
     for (cudaGraphExec_t &g : s->graph)
@@ -2803,6 +3047,14 @@ int fdtd_autotune(fdtd_solver *s, uint64_t trial_steps, int *layer_per_sm, int *
     CUDA_TRY(s, cudaEventCreate(&end));
     const bool timing = s->timing;
     s->timing = false;
+    // (The launched steps are tuned first; the resident stepper, where the grid may take it, is then
+    // timed against their best.)
+    struct Resident {
+        fdtd_solver *s;
+        bool allowed, chosen = false;
+        ~Resident() { s->resident = chosen; }
+    } resident{s, s->resident, s->resident};
+    s->resident = false;
     // Times trial_steps steps of the handle's present choice: one untimed dispatch, then the
     // faster of two timed ones (a single short pass was too noisy to rank close choices); ms < 0
     // when it could not run.
@@ -2913,6 +3165,17 @@ int fdtd_autotune(fdtd_solver *s, uint64_t trial_steps, int *layer_per_sm, int *
             best_layer = best.layer, best_special = best.special, best_concurrent = best.mode;
             s->concurrent = best.mode;
         }
+    }
+    if (rc == FDTD_OK && resident.allowed) {
+        recording = false;
+        s->layer_per_sm = best_layer, s->special_per_sm = best_special;
+        float least[2] = {-1.0f, -1.0f};
+        for (int repeat = 0; repeat < 6 && rc == FDTD_OK; ++repeat) {
+            s->resident = repeat % 2 != 0;
+            float ms;
+            if ((rc = trial(ms)) == FDTD_OK && (least[s->resident] < 0.0f || ms < least[s->resident])) least[s->resident] = ms;
+        }
+        resident.chosen = rc != FDTD_OK || least[1] < least[0];
     }
     s->timing = timing;
     cudaEventDestroy(start);
