@@ -327,27 +327,37 @@ __device__ __forceinline__ void layer_hat_cell(const AdjointTables &t, uint32_t 
     }
 }
 
-// The tables' products of a step whose Q^, L^, H^ waited in `pending` (layer_hat_cell), once its
-// forward factors are recorded.
+// The tables' products of `steps` steps whose Q^, L^, H^ waited (layer_hat_cell; step k's at waiting + 9 k
+// layers), with their forward factors: `traj` the first's, each next one's a step's factors before. The
+// steps' products are added in turn, one read and write of a cell's eighteen double sums for all of
+// them (their 288 bytes a cell are most of what a step of the tables' gradient moves).
 template <typename T>
-__global__ void __launch_bounds__(kBlock) layer_pending_kernel(const AdjointTables t, const T *pending, const T *traj,
-                                                               double *g) {
+__global__ void __launch_bounds__(kBlock) layer_pending_kernel(const AdjointTables t, const T *waiting, uint32_t steps,
+                                                               const T *traj, double *g) {
     const uint32_t c = blockIdx.x * kBlock + threadIdx.x;
     const uint32_t L = t.layers;
     if (c >= L) return;
     const T s = t.layer_scale ? (T)t.layer_scale[c] : (T)1;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const T q_hat = pending[(uint64_t)(3 * a) * L + c], lo_hat = pending[(uint64_t)(3 * a + 1) * L + c];
-        const T hi_hat = pending[(uint64_t)(3 * a + 2) * L + c];
-        const T *f = traj + (uint64_t)(6 * a) * L + c;
         double *gg = g + (uint64_t)(6 * a) * L + c;
-        gg[0] += (double)q_hat * (double)f[0];
-        gg[(uint64_t)1 * L] += -(double)q_hat * (double)s * (double)f[(uint64_t)1 * L];
-        gg[(uint64_t)2 * L] += (double)hi_hat * (double)f[(uint64_t)2 * L];
-        gg[(uint64_t)3 * L] += -(double)hi_hat * (double)f[(uint64_t)3 * L];
-        gg[(uint64_t)4 * L] += (double)lo_hat * (double)f[(uint64_t)4 * L];
-        gg[(uint64_t)5 * L] += -(double)lo_hat * (double)f[(uint64_t)5 * L];
+        double sum[6];
+#pragma unroll
+        for (int f = 0; f < 6; ++f) sum[f] = gg[(uint64_t)f * L];
+#pragma unroll 2
+        for (uint32_t k = 0; k < steps; ++k) {
+            const T *w = waiting + (uint64_t)k * 9 * L + c;
+            const T *f = traj - (uint64_t)k * kLayerFactors * L + (uint64_t)(6 * a) * L + c;
+            const T q_hat = w[(uint64_t)(3 * a) * L], lo_hat = w[(uint64_t)(3 * a + 1) * L], hi_hat = w[(uint64_t)(3 * a + 2) * L];
+            sum[0] += (double)q_hat * (double)f[0];
+            sum[1] += -(double)q_hat * (double)s * (double)f[(uint64_t)1 * L];
+            sum[2] += (double)hi_hat * (double)f[(uint64_t)2 * L];
+            sum[3] += -(double)hi_hat * (double)f[(uint64_t)3 * L];
+            sum[4] += (double)lo_hat * (double)f[(uint64_t)4 * L];
+            sum[5] += -(double)lo_hat * (double)f[(uint64_t)5 * L];
+        }
+#pragma unroll
+        for (int f = 0; f < 6; ++f) gg[(uint64_t)f * L] = sum[f];
     }
 }
 

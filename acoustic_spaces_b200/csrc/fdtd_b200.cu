@@ -28,6 +28,7 @@
 #include "fdtd_flow.cuh"
 #include "fdtd_kernels.cuh"
 #include "fdtd_resident.cuh"
+#include "fdtd_resident_adjoint.cuh"
 
 using namespace fdtd;
 
@@ -78,6 +79,11 @@ struct AdjointState {
     // The layer cells sorted by their coordinate along each axis in turn (x, then y, then z; each
     // a permutation of the cells) and each coordinate's first entry: the tables' sums by coordinate.
     const uint32_t *by_coord = nullptr, *coord_start = nullptr;
+    // The resident reverse stepper (fdtd_resident_adjoint.cuh), where the grid takes it: its interior's
+    // columns, its launch's blocks and where the shared memory's parts lie.
+    bool resident = false, clustered = false;
+    const uint2 *columns = nullptr;
+    uint32_t column_count = 0, blocks = 0, cells_at = 0, smem = 0;
 };
 
 }  // namespace
@@ -105,6 +111,7 @@ struct fdtd_solver {
     // on the 4 cm room's gradient: 0 and 8 took 99 ms for 200 reverse steps, 0 and 0 102.5 ms, and
     // any cap on the far rows more (106-257 ms).
     int adjoint_far_per_sm = 0, adjoint_near_per_sm = 8;
+    bool adjoint_launched = false;
     // How a step's kernels share the streams (fdtd_set_streams): 1, each kind on its own; 2, the
     // layer and then the special rows beside the sweep; 3, the special rows after the sweep, the
     // layer beside them; 0, all in turn (fdtd_autotune times them: where the special rows are many,
@@ -158,6 +165,7 @@ struct fdtd_solver {
     uint32_t resident_keep_layer = 0, resident_rows_at = 0, resident_layer_at = 0;
     const uint32_t *link_start = nullptr;
     const uint2 *row_links = nullptr;
+    std::vector<uint32_t> host_state_start;
     unsigned int *arrived = nullptr;
     void *gathered = nullptr;
     uint32_t gathered_count = 0;
@@ -870,6 +878,63 @@ int launch_steps(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
     return FDTD_OK;
 }
 
+// A launch of a resident kernel on the handle's stream: its blocks one cluster, or all of the GPU's at
+// once (they wait for one another: a cooperative launch holds them all or fails).
+cudaLaunchConfig_t together(const fdtd_solver *s, uint32_t blocks, int threads, uint32_t smem, bool clustered,
+                            cudaLaunchAttribute &attr) {
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(blocks), config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = smem;
+    config.stream = s->stream;
+    attr = cudaLaunchAttribute{};
+    if (clustered) {
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = blocks, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    } else {
+        attr.id = cudaLaunchAttributeCooperative;
+        attr.val.cooperative = 1;
+    }
+    config.attrs = &attr, config.numAttrs = 1;
+    return config;
+}
+
+template <class Kernel, class Args>
+int launch_together(fdtd_solver *s, Kernel kernel, uint32_t blocks, int threads, uint32_t smem, bool clustered, const Args &args) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t config = together(s, blocks, threads, smem, clustered, attr);
+    if (!clustered) CUDA_TRY(s, cudaMemsetAsync(s->arrived, 0, sizeof(unsigned int), s->stream));
+    CUDA_TRY(s, cudaLaunchKernelEx(&config, kernel, args));
+    return FDTD_OK;
+}
+
+// The blocks of a resident kernel whose tasks number `tasks` and whose block's shared memory smem(blocks)
+// gives: a cluster of 16 where two warps have a task at most, or else a block a multiprocessor. (A
+// cluster's barrier is the faster one, 2.3-2.5 us a step against 2.7-2.9 at 2,000 to 11,000 cells; from 50,000 cells its 16
+// multiprocessors are too few, 3.4-3.8 against 2.8-3.1.) False where they do not fit.
+template <class Kernel, class Smem>
+int choose_blocks(fdtd_solver *s, Kernel kernel, uint64_t tasks, int threads, Smem smem, uint32_t *blocks, bool *clustered,
+                  bool *fits) {
+    CUDA_TRY(s, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResidentSmem));
+    *clustered = false, *fits = true;
+    if (2 * tasks <= 16 * (uint64_t)(threads / 32) && smem(16) <= kResidentSmem) {
+        CUDA_TRY(s, cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchAttribute attr;
+        const cudaLaunchConfig_t config = together(s, 16, threads, smem(16), true, attr);
+        int clusters = 0;
+        CUDA_TRY(s, cudaOccupancyMaxActiveClusters(&clusters, kernel, &config));
+        if (clusters >= 1) {
+            *blocks = 16, *clustered = true;
+            return FDTD_OK;
+        }
+    }
+    *blocks = (uint32_t)s->sms;
+    int per_sm = 0;
+    const uint32_t bytes = smem(*blocks);
+    if (bytes <= kResidentSmem) CUDA_TRY(s, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, bytes));
+    *fits = per_sm >= 1;
+    return FDTD_OK;
+}
+
 // The steps by the resident stepper: pieces of at most gathered_steps steps a launch, each followed by
 // its probes' sums.
 template <typename T, bool WIDE, bool SCALED, bool COMP, bool LAYER>
@@ -905,24 +970,9 @@ int launch_resident(fdtd_solver *s, const float *d_signal, uint64_t steps, doubl
         a.steps = (uint32_t)count;
         a.clustered = s->resident_clustered ? 1 : 0;
         a.arrived = s->arrived, a.error = s->d_error;
-        cudaLaunchConfig_t config{};
-        config.gridDim = dim3(s->resident_blocks);
-        config.blockDim = dim3(kResidentThreads<T, WIDE, LAYER>);
-        config.dynamicSmemBytes = s->resident_smem;
-        config.stream = s->stream;
-        cudaLaunchAttribute attr{};
-        if (s->resident_clustered) {
-            attr.id = cudaLaunchAttributeClusterDimension;
-            attr.val.clusterDim.x = s->resident_blocks, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-        } else {
-            // The blocks wait for one another: all of them resident at once, or the launch fails.
-            attr.id = cudaLaunchAttributeCooperative;
-            attr.val.cooperative = 1;
-            CUDA_TRY(s, cudaMemsetAsync(s->arrived, 0, sizeof(unsigned int), s->stream));
-        }
-        config.attrs = &attr;
-        config.numAttrs = 1;
-        CUDA_TRY(s, cudaLaunchKernelEx(&config, resident_kernel<T, WIDE, SCALED, COMP, LAYER>, a));
+        const int launched = launch_together(s, resident_kernel<T, WIDE, SCALED, COMP, LAYER>, s->resident_blocks,
+                                             kResidentThreads<T, WIDE, LAYER>, s->resident_smem, s->resident_clustered, a);
+        if (launched != FDTD_OK) return launched;
         if (probes && s->gathered_count) {
             const int rc = sum_probes<T>(s, count, d_out + done, stride);
             if (rc != FDTD_OK) return rc;
@@ -942,17 +992,17 @@ int dispatch_run(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
 
 // The columns of quads of the interior, `planes` planes at most each: every run of planes that
 // holds interior cells, from its first, so that a column's first plane holds one.
-void interior_columns(const fdtd_solver *s, uint64_t planes, std::vector<uint2> &columns) {
+void interior_columns(const fdtd_solver *s, const std::vector<uint8_t> &types, uint64_t planes, std::vector<uint2> &columns) {
     columns.clear();
     const BulkArgs &bk = s->bulk;
-    if (s->host_types.empty()) return;
+    if (!s->interior || types.empty()) return;
     const uint64_t quads = s->pitch / 4, plane = s->pitch * s->ny;
     std::vector<uint32_t> masks(quads);
     for (uint64_t z0 = bk.z0; z0 < bk.z1; z0 += planes)
         for (uint64_t y = bk.y0; y < bk.y1; ++y) {
             std::fill(masks.begin(), masks.end(), 0u);
             for (uint64_t z = z0, end = std::min<uint64_t>(z0 + planes, bk.z1); z < end; ++z) {
-                const uint8_t *row = &s->host_types[plane * z + s->pitch * y];
+                const uint8_t *row = &types[plane * z + s->pitch * y];
                 for (uint64_t q = 0; q < quads; ++q) {
                     uint32_t four;
                     std::memcpy(&four, row + 4 * q, 4);
@@ -968,6 +1018,25 @@ void interior_columns(const fdtd_solver *s, uint64_t planes, std::vector<uint2> 
                 columns.push_back(make_uint2((uint32_t)(plane * (z0 + skip) + s->pitch * y + 4 * q), masks[q] >> (4 * skip)));
             }
         }
+}
+
+// The columns with as many planes each as leave every warp one task (a step is then one chain of
+// loads); where the tasks (`other` ones beside the columns') are more than the warps, the choice of the
+// fewest planes in turn a warp, two planes counted for a column's first loads. (Measured, 1, 2, 3, 4, 6 and 8
+// planes: the 576,000-cell box in double 5.83, 5.40, 5.69, 5.98, 6.05 and 7.00 us a step, the 864,000-cell wide hall
+// 7.46, 7.15, 6.52, 6.86, 7.68 and 8.10: the rule takes 3 for both.)
+void choose_columns(const fdtd_solver *s, const std::vector<uint8_t> &types, uint64_t other, uint64_t warps,
+                    std::vector<uint2> &columns) {
+    interior_columns(s, types, 1, columns);
+    const uint64_t quads = columns.size();
+    uint64_t best = 1;
+    double least = 1e300;
+    for (uint64_t planes = 1; planes <= kColumnPlanes; ++planes) {
+        const uint64_t rounds = (other + ((quads + planes - 1) / planes + 31) / 32 + warps - 1) / warps;
+        const double cost = (double)rounds * ((double)planes + 2.0);
+        if (cost < least) least = cost, best = planes;
+    }
+    if (best > 1) interior_columns(s, types, best, columns);
 }
 
 // Whether the grid takes the resident stepper: the bytes that its steps touch, against a limit.
@@ -997,28 +1066,14 @@ int set_up_resident(fdtd_solver *s, const std::vector<uint32_t> &link_start, con
     const int threads = kResidentThreads<T, WIDE, LAYER>;
     auto tasks = [](uint64_t n) { return (n + 31) / 32; };
     const uint64_t other = tasks(s->specials) + tasks(s->tables.layer_quads) + tasks(s->gathered_count);
-    // Planes a column: as few as leave every warp one task (a step is then one chain of loads);
-    // where the tasks are more than the warps, the choice of the fewest planes in turn a warp, two
-    // planes counted for a column's first loads.
-    const uint64_t warps = (uint64_t)s->sms * (threads / 32);
     std::vector<uint2> columns;
-    interior_columns(s, 1, columns);
-    uint64_t quads = columns.size(), best = 1;
-    double least = 1e300;
-    for (uint64_t planes = 1; planes <= kColumnPlanes; ++planes) {
-        const uint64_t rounds = (other + tasks((quads + planes - 1) / planes) + warps - 1) / warps;
-        const double cost = (double)rounds * ((double)planes + 2.0);
-        if (cost < least) least = cost, best = planes;
-    }
-    if (best > 1) interior_columns(s, best, columns);
+    choose_columns(s, s->host_types, other, (uint64_t)s->sms * (threads / 32), columns);
     int rc;
     if ((rc = upload(s, columns.data(), columns.size(), &s->columns))) return rc;
     s->column_count = (uint32_t)columns.size();
     const uint64_t all = other + tasks(columns.size());
-    // Blocks: one a multiprocessor, or a cluster's where its warps take the tasks a few each: its
-    // barrier is faster than one over the whole GPU.
     // The shared memory of a block's rows, if the largest block's fits.
-    auto stage = [&](uint32_t blocks) {
+    auto stage = [&](uint32_t blocks) -> uint32_t {
         uint32_t most = 0;
         for (uint32_t k = 0; k < blocks; ++k) {
             const uint32_t r0 = std::min<uint32_t>(share_of(s->tables.specials, k, blocks) * 32, s->tables.specials);
@@ -1035,35 +1090,12 @@ int set_up_resident(fdtd_solver *s, const std::vector<uint32_t> &link_start, con
         const uint32_t a_task = 9 * 128 * sizeof(T), left = kResidentSmem - std::min(kResidentSmem, s->resident_layer_at);
         const uint64_t a_block = (tasks(s->tables.layer_quads) + blocks - 1) / blocks;
         s->resident_keep_layer = (uint32_t)std::min<uint64_t>(a_block, left / a_task);
-        s->resident_smem = s->resident_layer_at + s->resident_keep_layer * a_task;
+        return s->resident_smem = s->resident_layer_at + s->resident_keep_layer * a_task;
     };
-    CUDA_TRY(s, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResidentSmem));
-    s->resident_blocks = (uint32_t)s->sms, s->resident_clustered = false;
+    bool fits = false;
+    if ((rc = choose_blocks(s, kernel, all, threads, stage, &s->resident_blocks, &s->resident_clustered, &fits)) != FDTD_OK) return rc;
+    if (!fits) return FDTD_OK;
     stage(s->resident_blocks);
-    if (2 * all <= 16 * (uint64_t)(threads / 32)) {
-        uint32_t blocks = 16;
-        CUDA_TRY(s, cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        for (; blocks; blocks = blocks == 16 ? 8 : 0) {
-            stage(blocks);
-            cudaLaunchConfig_t config{};
-            config.gridDim = dim3(blocks), config.blockDim = dim3(threads), config.dynamicSmemBytes = s->resident_smem;
-            cudaLaunchAttribute attr{};
-            attr.id = cudaLaunchAttributeClusterDimension;
-            attr.val.clusterDim.x = blocks, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-            config.attrs = &attr, config.numAttrs = 1;
-            int clusters = 0;
-            CUDA_TRY(s, cudaOccupancyMaxActiveClusters(&clusters, kernel, &config));
-            if (clusters < 1) continue;
-            s->resident_blocks = blocks, s->resident_clustered = true;
-            break;
-        }
-        if (!s->resident_clustered) stage(s->resident_blocks);
-    }
-    if (!s->resident_clustered) {
-        int per_sm = 0;
-        CUDA_TRY(s, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, s->resident_smem));
-        if (per_sm < 1) return FDTD_OK;
-    }
     void *p;
     if ((rc = zeros(s, sizeof(unsigned int), &p))) return rc;
     s->arrived = static_cast<unsigned int *>(p);
@@ -1504,7 +1536,8 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
     const uint64_t a_step = std::max<uint64_t>(1, s->gathered_count) * e;
     s->gathered_steps = std::min<uint64_t>(kGatheredSteps, std::max<uint64_t>(16, (32ull << 20) / a_step)) / 2 * 2;
     if ((rc = zeros(s, a_step * s->gathered_steps, &s->gathered))) return rc;
-    return resident ? set_up_resident_kind(s, link_start, state_start) : FDTD_OK;
+    s->host_state_start = std::move(state_start);
+    return resident ? set_up_resident_kind(s, link_start, s->host_state_start) : FDTD_OK;
 }
 
 void release(fdtd_solver *s) {
@@ -1903,6 +1936,45 @@ struct Owned {
     }
 };
 
+template <typename T, bool WIDE, bool SCALED, bool LAYER>
+int set_up_reverse(fdtd_solver *s, const AdjointLists &l) {
+    AdjointState &a = s->adjoint;
+    auto tasks = [](uint64_t n) { return (n + 31) / 32; };
+    const uint64_t other = tasks(s->specials) + tasks(l.cells.size()) + tasks(s->layers);
+    std::vector<uint2> columns;
+    choose_columns(s, l.types, other, (uint64_t)s->sms * (kReverseThreads / 32), columns);
+    auto smem = [&](uint32_t blocks) -> uint32_t {
+        uint64_t rows = 0, cells = 0;
+        const uint32_t K = (uint32_t)s->specials, C = (uint32_t)l.cells.size();
+        for (uint32_t k = 0; k < blocks; ++k) {
+            const uint32_t r0 = std::min(share_of(K, k, blocks) * 32, K), r1 = std::min(share_of(K, k + 1, blocks) * 32, K);
+            rows = std::max<uint64_t>(rows, AdjointStage<T>::bytes(r1 - r0, l.reader_start[r1] - l.reader_start[r0],
+                                                                   s->host_state_start[r1] - s->host_state_start[r0]));
+            const uint32_t c0 = std::min(share_of(C, k, blocks) * 32, C), c1 = std::min(share_of(C, k + 1, blocks) * 32, C);
+            cells = std::max<uint64_t>(cells, WholeStage<T>::bytes(c1 - c0, l.starts[c1] - l.starts[c0]));
+        }
+        a.cells_at = (uint32_t)((rows + 127) / 128 * 128);
+        return a.smem = (uint32_t)std::min<uint64_t>(a.cells_at + cells, UINT32_MAX);
+    };
+    bool fits = false;
+    int rc;
+    auto kernel = reverse_kernel<T, WIDE, SCALED, LAYER>;
+    if ((rc = choose_blocks(s, kernel, other + tasks(columns.size()), kReverseThreads, smem, &a.blocks, &a.clustered, &fits)) != FDTD_OK)
+        return rc;
+    if (!fits) return FDTD_OK;
+    smem(a.blocks);
+    if ((rc = upload(s, columns.data(), columns.size(), &a.columns))) return rc;
+    a.column_count = (uint32_t)columns.size();
+    a.resident = true;
+    return FDTD_OK;
+}
+
+// The reverse stepper's instantiation for the grid: stencil, speed field, matched layer.
+#define FDTD_REVERSE(CALL)                                                                                  \
+    (s->wide ? (s->scaled ? CALL(true, true, false) : CALL(true, false, false))                             \
+             : (s->layers ? (s->scaled ? CALL(false, true, true) : CALL(false, false, true))                \
+                          : (s->scaled ? CALL(false, true, false) : CALL(false, false, false))))
+
 // The handle's adjoint, set up on first use and kept; every copy and clear has ended on return.
 int set_up_adjoint(fdtd_solver *s) {
     if (s->adjoint_ready) return FDTD_OK;
@@ -1911,6 +1983,13 @@ int set_up_adjoint(fdtd_solver *s) {
     if ((rc = adjoint_lists(s, lists))) return rc;
     Owned owned{s};
     if ((rc = place_adjoint(s, lists, owned, s->adjoint))) return rc;
+    if (s->resident) {
+#define SET_F(W, S, L) set_up_reverse<float, W, S, L>(s, lists)
+#define SET_D(W, S, L) set_up_reverse<double, W, S, L>(s, lists)
+        if ((rc = s->precision == FDTD_FP64 ? FDTD_REVERSE(SET_D) : FDTD_REVERSE(SET_F)) != FDTD_OK) return rc;
+#undef SET_F
+#undef SET_D
+    }
     CUDA_TRY(s, cudaDeviceSynchronize());  // the clears (default stream) and copies (handle's stream)
     s->adjoint_reader_row = std::move(lists.reader_row);
     s->adjoint_reader_base = std::move(lists.reader_base);
@@ -2025,9 +2104,14 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
     if ((rc = scratch.take(sizeof(double) * std::max<uint64_t>(1, P) * steps, &p))) return rc;
     double *d_dloss = static_cast<double *>(p);
     if (P) CUDA_TRY(s, cudaMemcpyAsync(d_dloss, dloss, sizeof(double) * P * steps, cudaMemcpyHostToDevice, s->stream));
-    if ((rc = scratch.take(e * K * (segment + 2), &p))) return rc;
+    // The resident reverse stepper takes the segments' steps in a launch each, and with every level on
+    // the tape reads them there.
+    const bool resident = graphs && s->resident && adj.resident && !s->adjoint_launched && !s->timing;
+    const bool from_tape = resident && holds_tape(s, signal, steps, segment) && s->tape_traj;
+    const uint64_t kept_levels = from_tape ? 0 : segment + 2;
+    if ((rc = scratch.take(e * K * kept_levels, &p))) return rc;
     T *traj_u = static_cast<T *>(p);
-    if ((rc = scratch.take(e * S * (segment + 2), &p))) return rc;
+    if ((rc = scratch.take(e * S * kept_levels, &p))) return rc;
     T *traj_w = static_cast<T *>(p);
     if ((rc = scratch.take(sizeof(double) * std::max<uint64_t>(1, P) * segment, &p))) return rc;
     double *d_out = static_cast<double *>(p);
@@ -2047,7 +2131,8 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
     const uint64_t Lc = s->layers;
     const bool tangent = Lc && s->tangent;  // along a tangent of the tables, in place of the tables
     const bool tables = Lc && s->gradient_tables && !tangent;
-    T *traj_layer = nullptr;
+    T *traj_layer = nullptr, *waiting = nullptr;
+    uint64_t waiting_steps = 0;
     double *g_layer = nullptr, *table_sums = nullptr;
     const uint64_t coords = s->nx + s->ny + s->nz;
     if (tables) {
@@ -2057,6 +2142,12 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
         g_layer = static_cast<double *>(p);
         if ((rc = scratch.take(sizeof(double) * 6 * coords, &p))) return rc;
         table_sums = static_cast<double *>(p);
+        if (resident) {
+            // The Q^, L^, H^ of a launch's steps: 128 MiB of them at most, 4 steps at least.
+            waiting_steps = std::min<uint64_t>(segment, std::max<uint64_t>(4, (128ull << 20) / (9 * e * Lc)));
+            if ((rc = scratch.take(9 * e * Lc * waiting_steps, &p))) return rc;
+            waiting = static_cast<T *>(p);
+        }
     }
     // The forward pass from rest, keeping checkpoints[m] = the state at the start of segment m+1;
     // or, when the handle holds the tape of a run of this drive with these segments, its states.
@@ -2133,7 +2224,53 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
         s->record_u = s->record_w = s->record_layer = s->record_tangent = nullptr, s->record_probes = true;
         return r;
     };
+    // Steps first, first - 1, ... (`count` of them) by the resident reverse stepper, the trajectory's level
+    // of step 0 at u, w, and dL/dy's column of step 0 at d.
+    auto reverse_resident = [&](uint64_t first, uint64_t count, const T *u, const T *w, const double *d, uint64_t stride) -> int {
+        ReverseArgs<T> a{};
+        a.t = t;
+        a.sweep.g.pitch = s->tables.pitch, a.sweep.g.plane = s->tables.plane;
+        a.sweep.scale = s->scale_device;
+        a.sweep.columns = adj.columns, a.sweep.column_count = adj.column_count;
+        a.sweep.axial = s->bulk.axial, a.sweep.diagonal = s->bulk.diagonal;
+        a.sweep.centre = s->bulk.centre, a.sweep.total = s->bulk.total;
+        for (int k = 0; k < 2; ++k) {
+            const int from = k ? 1 - x : x;
+            a.lam[k] = static_cast<T *>(adj.lam[from]), a.om[k] = static_cast<T *>(adj.om[from]);
+            a.tilde[k] = static_cast<T *>(adj.tilde[from]), a.hat[k] = static_cast<T *>(adj.hat[from]);
+        }
+        a.traj_u = u, a.traj_w = w, a.dloss = d, a.stride = stride;
+        a.first = (uint32_t)first, a.steps = (uint32_t)count;
+        a.g_cb = g[0], a.g_ci = g[1], a.g_now = g[2], a.g_before = g[3], a.g_gain = g[4];
+        a.next = LayerNext<T>{nullptr, static_cast<T *>(adj.carried), tables || tangent ? static_cast<T *>(adj.pending) : nullptr,
+                              nullptr, nullptr, tangent ? tan_base : nullptr, 0};
+        a.waiting = waiting;
+        a.tangent_factors = (uint32_t)Tf;
+        a.cells_at = adj.cells_at, a.clustered = adj.clustered ? 1 : 0;
+        a.arrived = s->arrived, a.error = s->d_error;
+#define LAUNCH(W, S, L) launch_together(s, reverse_kernel<T, W, S, L>, adj.blocks, kReverseThreads, adj.smem, adj.clustered, a)
+        return FDTD_REVERSE(LAUNCH);
+#undef LAUNCH
+    };
     auto reverse = [&](uint64_t count) -> int {
+        if (resident && !tables) return reverse_resident(count - 1, count, traj_u, traj_w, seg_dloss, segment);
+        // (With the tables, in launches of the steps whose Q^, L^, H^ fit the workspace, their products after
+        // each; the last step's wait for the segment before, layer_pending_kernel there.)
+        for (uint64_t done = 0; resident && done < count;) {
+            const uint64_t n = std::min(count - done, waiting_steps), first = count - 1 - done;
+            const int r = reverse_resident(first, n, traj_u, traj_w, seg_dloss, segment);
+            if (r != FDTD_OK) return r;
+            const uint64_t products = std::min(n, first);  // (step 0 has its factors in the segment before)
+            if (products) layer_pending_kernel<T><<<layer_blocks, kBlock, 0, s->stream>>>(
+                    t, waiting, (uint32_t)products, traj_layer + (first - 1) * kLayerFactors * Lc, g_layer);
+            CUDA_TRY(s, cudaGetLastError());
+            if (n & 1) x = 1 - x;
+            done += n;
+            if (done == count) {
+                if (count & 1) x = 1 - x;  // (the caller turns the levels after the segment)
+                return FDTD_OK;
+            }
+        }
         int xx = x;
         for (uint64_t m = count; m-- > 0;) {
             T *lam_next = static_cast<T *>(adj.lam[xx]), *lam_out = static_cast<T *>(adj.lam[1 - xx]);
@@ -2211,7 +2348,7 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
     }
     auto run = [&](int which, int key, auto &&body, uint64_t count) -> int {
         // (The resident stepper's recomputation is a launch or two: nothing to capture.)
-        if (!graphs || count != segment || segments == 1 || (which == 0 && s->resident && !s->timing)) return body(count);
+        if (!graphs || count != segment || segments == 1 || (which == 0 ? s->resident && !s->timing : resident)) return body(count);
         cudaGraphExec_t &exec = s->grad_graph[which][key];
         if (!exec) {
             const bool timing = s->timing;
@@ -2239,7 +2376,11 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
         layer_tangent_flush_kernel<T><<<layer_blocks, kBlock, 0, s->stream>>>((uint32_t)Lc, static_cast<T *>(adj.carried),
                                                                               tan_acc);
     };
-    for (uint64_t k = segments; k-- > 0;) {
+    const bool whole = from_tape && !tangent;  // nothing between the segments: one launch takes them all
+    if (whole && (rc = reverse_resident(steps - 1, steps, static_cast<const T *>(s->tape_u), static_cast<const T *>(s->tape_w),
+                                        d_dloss, steps)) != FDTD_OK)
+        return rc;
+    for (uint64_t k = whole ? 0 : segments; k-- > 0;) {
         const uint64_t s0 = k * segment, s1 = std::min(steps, s0 + segment), count = s1 - s0;
         if (tangent) {
             // Where the segment's factors start; and the products of its last step, whose Q^, L^,
@@ -2254,6 +2395,14 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
                     t, static_cast<const T *>(adj.pending), static_cast<const T *>(s->tape_t) + (s0 + count - 1) * Tf,
                     tan_acc);
                 CUDA_TRY(s, cudaGetLastError());
+            }
+            if (resident) {
+                if ((rc = reverse_resident(count - 1, count, static_cast<const T *>(s->tape_u) + s0 * K,
+                                           static_cast<const T *>(s->tape_w) + s0 * S, d_dloss + s0, steps)) != FDTD_OK)
+                    return rc;
+                if (tangent) flush_tangent();
+                if (count & 1) x = 1 - x;
+                continue;
             }
             // The segment's levels s0 .. s1+1 from the tape, into the segment's trajectory buffers.
             CUDA_TRY(s, cudaMemcpyAsync(traj_u, static_cast<const T *>(s->tape_u) + s0 * K, e * K * (count + 2),
@@ -2292,7 +2441,7 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
         // left waiting: its factors are recorded now.
         if (tables && k + 1 < segments) {
             layer_pending_kernel<T><<<layer_blocks, kBlock, 0, s->stream>>>(
-                t, static_cast<const T *>(adj.pending), traj_layer + (count - 1) * kLayerFactors * Lc, g_layer);
+                t, static_cast<const T *>(adj.pending), 1, traj_layer + (count - 1) * kLayerFactors * Lc, g_layer);
             CUDA_TRY(s, cudaGetLastError());
         }
         if (tangent && k + 1 < segments) {
@@ -3006,6 +3155,7 @@ int fdtd_set_adjoint_launch(fdtd_solver *s, int far_per_sm, int near_per_sm) {
     DeviceGuard guard(s->device);
     CUDA_TRY(s, cudaStreamSynchronize(s->stream));
     s->adjoint_far_per_sm = far_per_sm, s->adjoint_near_per_sm = near_per_sm;
+    s->adjoint_launched = true;  // (the caller chooses the launches: the reverse steps are launched)
     Kept{s}.drop_graphs();  // the gradient's graphs hold the old launches
     return FDTD_OK;
 }

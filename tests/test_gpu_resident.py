@@ -118,3 +118,53 @@ def test_gpu_handles_step_from_two_threads():
         t.join()
     for k in (0, 1):
         assert all(np.array_equal(y, alone[k]) for y in got[k])
+
+
+# ---- the reverse steps -------------------------------------------------------------------------
+
+
+def _gradients(layout, precision, steps, segment, tape, tables=True, tangent=None, launched=False):
+    solver = B200WaveSolver(layout, precision=precision)
+    if launched:
+        solver.set_adjoint_launch(0, 8)
+    if tangent is not None:
+        solver.set_layer_tangent(tangent)
+    if tape:
+        solver.set_tape(segment, layer_tables=tables)
+    drive = _drive(steps, 4)
+    y = solver.run(drive)
+    solver.reset()
+    dloss = y * np.linspace(0.5, 1.5, steps)
+    return solver.gradient(drive, dloss, segment=segment, layer_tables=tables)
+
+
+def _same(a, b):
+    assert a.keys() == b.keys()
+    for key in a:
+        assert np.array_equal(a[key], b[key]), key
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("tape", [False, True])
+@pytest.mark.parametrize("shape, speed", [((12, 9, 11), None), ((13, 16, 13), 0.9), ((60, 41, 30), None), ((90, 77, 40), 0.97)])
+def test_gpu_resident_reverse_steps_equal_the_launched_ones(shape, speed, tape, precision):
+    layout = _box(shape, speed=speed)
+    args = (layout, precision, 61, 20, tape)
+    _same(_gradients(*args), _gradients(*args, launched=True))
+
+
+@pytest.mark.parametrize("name", ["resonant19", "speed19"])
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_gpu_resident_reverse_wide_steps_equal_the_launched_ones(name, precision):
+    layout = layouts.stack([load_golden(name)[0]] * 4, across=2).layout
+    _same(_gradients(layout, precision, 50, 25, True), _gradients(layout, precision, 50, 25, True, launched=True))
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("kind", ["tables", "walls", "tangent"])
+@pytest.mark.parametrize("cell", [0.3, 0.2])
+def test_gpu_resident_reverse_layers_equal_the_launched_ones(cell, kind, precision):
+    layout = layouts.polyhedral_room(2, cell=cell, receivers=3, steps=1).built.layout
+    tangent = layouts.damping_tangent(layout, layouts.LAYER_CELLS, layouts.LAYER_DAMPING) if kind == "tangent" else None
+    args = (layout, precision, 130, 50, True, kind == "tables", tangent)
+    _same(_gradients(*args), _gradients(*args, launched=True))
