@@ -165,6 +165,7 @@ struct fdtd_solver {
     uint32_t resident_keep_layer = 0, resident_rows_at = 0, resident_layer_at = 0;
     const uint32_t *link_start = nullptr;
     const uint2 *row_links = nullptr;
+    void *resident_work = nullptr;  // the layer's state of the tasks that shared memory does not hold
     std::vector<uint32_t> host_state_start;
     unsigned int *arrived = nullptr;
     void *gathered = nullptr;
@@ -958,6 +959,7 @@ int launch_resident(fdtd_solver *s, const float *d_signal, uint64_t steps, doubl
         a.signal = d_signal + done;
         a.link_start = s->link_start, a.links = s->row_links, a.staged = s->resident_staged ? 1 : 0;
         a.keep_layer = s->resident_keep_layer, a.rows_at = s->resident_rows_at, a.layer_at = s->resident_layer_at;
+        a.layer_work = static_cast<T *>(s->resident_work);
         a.coefs[0] = (uint32_t)s->pitch + 2, a.coefs[1] = (uint32_t)s->ny + 1, a.coefs[2] = (uint32_t)s->nz + 1;
         a.gathered = static_cast<T *>(s->gathered), a.gathered_count = probes ? s->gathered_count : 0;
         if (s->record_u) {
@@ -1097,6 +1099,10 @@ int set_up_resident(fdtd_solver *s, const std::vector<uint32_t> &link_start, con
     if (!fits) return FDTD_OK;
     stage(s->resident_blocks);
     void *p;
+    if (LAYER) {
+        if ((rc = zeros(s, tasks(s->tables.layer_quads) * 9 * 128 * sizeof(T), &p))) return rc;
+        s->resident_work = p;
+    }
     if ((rc = zeros(s, sizeof(unsigned int), &p))) return rc;
     s->arrived = static_cast<unsigned int *>(p);
     s->resident = true;

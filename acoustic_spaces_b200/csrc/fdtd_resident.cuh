@@ -33,10 +33,11 @@ struct ResidentArgs {
     const uint32_t *link_start;
     const uint2 *links;
     uint32_t staged;
-    // The layer's coefficients and, of as many tasks a block as fit (keep_layer), its state kept in
+    // The layer's coefficients and, of as many tasks a block as fit (keep_layer), its state are kept in
     // shared memory too: where the rows (after the coefficients) and the state begin, and the
     // coefficients' counts along x, y and z.
     uint32_t keep_layer, rows_at, layer_at, coefs[3];
+    T *layer_work;  // the other tasks' state, in the same form (nine quads a quad)
     // The probes' cells of every step, gathered in their order (summed by probe_sum_kernel).
     T *gathered;
     uint32_t gathered_count;
@@ -381,10 +382,13 @@ __global__ void __launch_bounds__(kResidentThreads<T, WIDE, LAYER>, 1)
             m.w[j] = p.w[0][s0 + j], m.w[m.states + j] = p.w[1][s0 + j];
         }
     }
-    // The layer's state: nine quads a quad, 32 of them (a task's) together, slot by slot, each its own
-    // thread's alone; and its coefficients.
-    T *kept_layer = reinterpret_cast<T *>(smem + p.layer_at) + 4 * lane;
-    const uint32_t kept_tasks = LAYER ? min(p.keep_layer, layer) : 0u;
+    // The layer's state: nine quads a quad, its own copy of both faces on each axis as the reference
+    // keeps it, 32 quads (a task's) together, slot by slot, each its own thread's alone and updated in
+    // place, in shared memory or, past what fits there, in the workspace; and its coefficients.
+    auto kept_at = [&](uint32_t t) {
+        return t < p.keep_layer ? reinterpret_cast<T *>(smem + p.layer_at) + t * 9 * 128 + 4 * lane
+                                : p.layer_work + (uint64_t)(layer0 + t) * 9 * 128 + 4 * lane;
+    };
     const float4 *coef[3] = {};
     if (LAYER) {
         float4 *at = reinterpret_cast<float4 *>(smem);
@@ -393,14 +397,14 @@ __global__ void __launch_bounds__(kResidentThreads<T, WIDE, LAYER>, 1)
             for (uint32_t x = threadIdx.x; x < p.coefs[a]; x += kThreads) at[x] = g.layer_coef[a][x];
             coef[a] = at, at += p.coefs[a];
         }
-        for (uint32_t t = warp; t < kept_tasks; t += kWarps) {
+        for (uint32_t t = warp; t < layer; t += kWarps) {
             const uint32_t q = (layer0 + t) * 32 + lane;
             if (q >= g.layer_quads) continue;
             const uint4 d = g.layer_quad[q];
             if (!(d.w & 15u)) continue;
             LayerState<T> s;
             load_layer(p.layer[1], g.layer_lanes, q, d, s);
-            keep_state(kept_layer + t * 9 * 128, s);
+            keep_state(kept_at(t), s);
         }
     }
     __syncthreads();
@@ -433,7 +437,6 @@ __global__ void __launch_bounds__(kResidentThreads<T, WIDE, LAYER>, 1)
         Fields<T> f{};
         f.b = cur ? p.u[1] : p.u[0], f.a = cur ? p.u[0] : p.u[1];
         f.wb = cur ? p.w[1] : p.w[0], f.wa = cur ? p.w[0] : p.w[1], f.d = p.d;
-        f.cell_old = cur ? p.layer[1] : p.layer[0], f.cell_new = cur ? p.layer[0] : p.layer[1];
         f.signal = p.signal + k;
         if (p.traj_u) f.traj_u = p.traj_u + (uint64_t)k * g.specials, f.traj_w = p.traj_w + (uint64_t)k * p.states;
         if (LAYER && p.traj_layer) f.traj_layer = p.traj_layer + (uint64_t)k * 18 * g.layers;
@@ -461,17 +464,11 @@ __global__ void __launch_bounds__(kResidentThreads<T, WIDE, LAYER>, 1)
             } else if (LAYER && t < rows + layer) {
                 const uint32_t q = (layer0 + t - rows) * 32 + lane;
                 if (!(e.w & 15u)) continue;
-                T *kept = kept_layer + (t - rows) * 9 * 128;
+                T *kept = kept_at(t - rows);
                 LayerState<T> s;
-                if (t - rows < kept_tasks)
-                    kept_state(kept, s);
-                else
-                    load_layer(f.cell_old, g.layer_lanes, q, e, s);
+                kept_state(kept, s);
                 step_layer<T, SCALED, COMP, false>(g, f, coef, q, e, s);
-                if (t - rows < kept_tasks)
-                    keep_state(kept, s);
-                else
-                    store_layer<false>(f.cell_new, g.layer_lanes, q, e, s);
+                keep_state(kept, s);
             } else if (t < rows + layer + reads) {
                 const uint32_t c = (reads0 + t - rows - layer) * 32 + lane;
                 if (c < p.gathered_count) p.gathered[(uint64_t)k * p.gathered_count + c] = f.b[e.x];
@@ -492,13 +489,13 @@ __global__ void __launch_bounds__(kResidentThreads<T, WIDE, LAYER>, 1)
     if (LAYER) {
         // (into the set that is the current one after the launch's steps)
         T *to = p.steps & 1u ? p.layer[0] : p.layer[1];
-        for (uint32_t t = warp; t < kept_tasks; t += kWarps) {
+        for (uint32_t t = warp; t < layer; t += kWarps) {
             const uint32_t q = (layer0 + t) * 32 + lane;
             if (q >= g.layer_quads) continue;
             const uint4 d = g.layer_quad[q];
             if (!(d.w & 15u)) continue;
             LayerState<T> s;
-            kept_state(kept_layer + t * 9 * 128, s);
+            kept_state(kept_at(t), s);
             store_layer<false>(to, g.layer_lanes, q, d, s);
         }
     }

@@ -66,7 +66,7 @@ def test_gpu_wide_grids_step_as_the_oracle_does(count, precision):
 
 
 @pytest.mark.parametrize("precision", ["fp32", "fp64", "fp32c"])
-@pytest.mark.parametrize("cell", [0.3, 0.21, 0.16])
+@pytest.mark.parametrize("cell", [0.3, 0.21, 0.16, 0.13])  # (0.13: more state than shared memory holds)
 def test_gpu_layers_step_as_the_oracle_does(cell, precision):
     w = layouts.polyhedral_room(2, cell=cell, receivers=3, steps=1)
     _equal(w.built.layout, _drive(45), [0, 20, 45], precision)
