@@ -50,12 +50,12 @@ constexpr int kSteps[18][3] = {
 constexpr uint64_t kPitchCells = 16;  // rows padded to a multiple of 16 cells
 constexpr uint64_t kFineX = 32, kFineY = 16;  // the blocks tile_list counts interior cells in
 constexpr uint64_t kGraphSteps = 64;  // steps of fdtd_run's captured chunk (even: the roles return)
-// Grids of at least this many (pitched) cells step by direct launches in fdtd_run: their steps are
-// long enough (a quarter of a millisecond and more) that launching costs nothing, and replaying a
-// captured graph measured 8 % slower than the launches on the 47M-cell room (the streams
-// overlapped less). Smaller grids replay the graph: below some 10M cells a step's launches and
-// event waits cost as much host time as the step takes on the device.
-constexpr uint64_t kGraphCells = 1ull << 25;
+// Grids of at least this many (pitched) cells step by direct launches in fdtd_run, as fdtd_autotune times
+// them: a step takes 30 us and more, its launches less. Replaying a captured graph measured 8 % slower on
+// the 47M-cell room, and on the 17M-cell outdoor grid 2 % faster or 20 % slower (82 or 103 against 85 us a step)
+// with the choice tuned on direct launches. Smaller grids that do not take the resident stepper replay
+// the graph: a step's launches and event waits cost as much host time as it takes on the device.
+constexpr uint64_t kGraphCells = 1ull << 23;
 constexpr uint32_t kResidentSmem = 216 * 1024;  // shared memory a block of the resident stepper takes at most
 constexpr uint64_t kGatheredSteps = 1024;  // steps the probes' cells are gathered over at most (even)
 
@@ -962,7 +962,7 @@ int launch_resident(fdtd_solver *s, const float *d_signal, uint64_t steps, doubl
         a.link_start = s->link_start, a.links = s->row_links, a.staged = s->resident_staged ? 1 : 0;
         a.keep_layer = s->resident_keep_layer, a.rows_at = s->resident_rows_at, a.layer_at = s->resident_layer_at;
         a.layer_work = static_cast<T *>(s->resident_work);
-        a.coefs[0] = (uint32_t)s->pitch + 2, a.coefs[1] = (uint32_t)s->ny + 1, a.coefs[2] = (uint32_t)s->nz + 1;
+        a.coefs[0] = 4 * s->tables.x_quads, a.coefs[1] = (uint32_t)s->ny + 1, a.coefs[2] = (uint32_t)s->nz + 1;
         a.gathered = static_cast<T *>(s->gathered), a.gathered_count = probes ? s->gathered_count : 0;
         if (s->record_u) {
             a.traj_u = static_cast<T *>(s->record_u) + (done + s->record_offset) * s->specials;
@@ -1056,7 +1056,7 @@ bool takes_resident(const fdtd_solver *s, const fdtd_layout *L) {
     if (L->flow_count) return false;
     const uint64_t e = s->precision == FDTD_FP64 ? 8 : 4, MB = 1000 * 1000;
     const uint64_t a_cell = 2 * e + (s->precision == FDTD_FP32_COMPENSATED ? e : 0) + (s->scaled ? 4 : 0);
-    const uint64_t touched = a_cell * s->n_device + 2 * kLayerSlots * e * L->layer_count;
+    const uint64_t touched = a_cell * s->air + 2 * kLayerSlots * e * L->layer_count;
     if (e == 4) return touched <= 100 * MB;
     return touched <= (s->wide ? 50 * MB : (L->layer_count ? 80 * MB : 190 * MB));
 }
@@ -1065,7 +1065,7 @@ bool takes_resident(const fdtd_solver *s, const fdtd_layout *L) {
 template <typename T, bool WIDE, bool SCALED, bool COMP, bool LAYER>
 int set_up_resident(fdtd_solver *s, const std::vector<uint32_t> &link_start, const std::vector<uint32_t> &state_start) {
     s->resident = false;
-    if (LAYER && 16 * (s->pitch + s->ny + s->nz + 4) > kResidentSmem) return FDTD_OK;  // (a grid of lines)
+    if (LAYER && 16 * (s->pitch + s->ny + s->nz + 6) > kResidentSmem) return FDTD_OK;  // (a grid of lines)
     auto kernel = resident_kernel<T, WIDE, SCALED, COMP, LAYER>;
     const int threads = kResidentThreads<T, WIDE, LAYER>;
     auto tasks = [](uint64_t n) { return (n + 31) / 32; };
@@ -1087,7 +1087,7 @@ int set_up_resident(fdtd_solver *s, const std::vector<uint32_t> &link_start, con
         }
         // The layer's coefficients first, then the rows, then the state of as many of the layer's tasks
         // as fit beside them (nine quads a quad).
-        const uint32_t coefs = LAYER ? 16 * (uint32_t)(s->pitch + 2 + s->ny + 1 + s->nz + 1) : 0;
+        const uint32_t coefs = LAYER ? 16 * (uint32_t)(s->pitch + 4 + s->ny + 1 + s->nz + 1) : 0;
         s->resident_staged = coefs + most <= kResidentSmem;
         s->resident_rows_at = (coefs + 127u) / 128u * 128u;
         s->resident_layer_at = s->resident_rows_at + (s->resident_staged ? (most + 127u) / 128u * 128u : 0);
@@ -1503,14 +1503,21 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
             if ((rc = zeros(s, e * kLayerSlots * g.layer_lanes, &s->layer_state[k]))) return rc;
         const uint64_t len[3] = {nx + 1, ny + 1, nz + 1};
         for (int axis = 0; axis < 3; ++axis) {
-            // (Along x padded to the pitch: a quad's lanes beyond the grid read entries too.)
-            std::vector<float4> packed(axis == 0 ? s->pitch + 2 : len[axis], make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+            std::vector<float4> packed(len[axis]);
             for (uint64_t x = 0; x < len[axis]; ++x)
                 packed[x] = make_float4(L->keep[2 * axis][x], L->push[2 * axis][x], L->keep[2 * axis + 1][x],
                                         L->push[2 * axis + 1][x]);
             const float4 *p4;
-            if ((rc = upload(s, packed.data(), packed.size(), &p4))) return rc;
+            if ((rc = upload(s, packed.data(), len[axis], &p4))) return rc;
             g.layer_coef[axis] = p4;
+            if (axis == 0) {
+                // Along x by quads (entry 4 q + j at j x_quads + q; zero beyond the grid).
+                g.x_quads = (uint32_t)(s->pitch / 4 + 1);
+                std::vector<float4> by_quad(4 * g.x_quads, make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+                for (uint64_t x = 0; x < len[0]; ++x) by_quad[(x % 4) * g.x_quads + x / 4] = packed[x];
+                if ((rc = upload(s, by_quad.data(), by_quad.size(), &p4))) return rc;
+                g.layer_coef_x = p4;
+            }
         }
         if (s->scaled) {
             if ((rc = upload(s, L->layer_scale, Lc, &fp))) return rc;
@@ -3205,13 +3212,13 @@ int fdtd_autotune(fdtd_solver *s, uint64_t trial_steps, int *layer_per_sm, int *
     CUDA_TRY(s, cudaEventCreate(&end));
     const bool timing = s->timing;
     s->timing = false;
-    // (The launched steps are tuned first; the resident stepper, where the grid may take it, is then
-    // timed against their best.)
+    // (The launched steps are tuned; whether steps are launched is the grid's, takes_resident: trials on
+    // fields at rest rank the resident stepper too well, a 14M-cell stack 62 us a step in them and 75 in a run.)
     struct Resident {
         fdtd_solver *s;
-        bool allowed, chosen = false;
-        ~Resident() { s->resident = chosen; }
-    } resident{s, s->resident, s->resident};
+        bool kept;
+        ~Resident() { s->resident = kept; }
+    } resident{s, s->resident};
     s->resident = false;
     // Times trial_steps steps of the handle's present choice: one untimed dispatch, then the
     // faster of two timed ones (a single short pass was too noisy to rank close choices); ms < 0
@@ -3323,17 +3330,6 @@ int fdtd_autotune(fdtd_solver *s, uint64_t trial_steps, int *layer_per_sm, int *
             best_layer = best.layer, best_special = best.special, best_concurrent = best.mode;
             s->concurrent = best.mode;
         }
-    }
-    if (rc == FDTD_OK && resident.allowed) {
-        recording = false;
-        s->layer_per_sm = best_layer, s->special_per_sm = best_special;
-        float least[2] = {-1.0f, -1.0f};
-        for (int repeat = 0; repeat < 6 && rc == FDTD_OK; ++repeat) {
-            s->resident = repeat % 2 != 0;
-            float ms;
-            if ((rc = trial(ms)) == FDTD_OK && (least[s->resident] < 0.0f || ms < least[s->resident])) least[s->resident] = ms;
-        }
-        resident.chosen = rc != FDTD_OK || least[1] < least[0];
     }
     s->timing = timing;
     cudaEventDestroy(start);

@@ -525,6 +525,11 @@ struct Tables {
     const uint32_t *layer_cells;
     const float *layer_scale;
     const float4 *layer_coef[3];
+    // The same along x by quads, entry 4 q + j at j x_quads + q: a warp's quads beside one another read
+    // whole lines of it (at 4 q + j they read a quarter of each, and the layer's kernel waited for the
+    // cache: 92.7 us on the 4 cm room).
+    uint32_t x_quads;
+    const float4 *layer_coef_x;
     // The quads that hold layer cells or cells below one (four adjacent cells of a row each, from a
     // multiple of four; ascending): {the quad's pitched index, the quads a row and a plane before it,
     // bits 0-3: its layer cells, bits 4 a + 4 ..: those whose cell below along axis a is in the layer
@@ -844,10 +849,9 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const uint32_t at = a == 0 ? x : (a == 1 ? y : z);
-        // (The table along x is padded to the pitch: a quad's lanes beyond the grid read it too.)
         float4 c[5];
 #pragma unroll
-        for (int j = 0; j < (a == 0 ? 5 : 2); ++j) c[j] = coef[a][at + j];
+        for (int j = 0; j < (a == 0 ? 5 : 2); ++j) c[j] = a == 0 ? coef[0][(j % 4) * g.x_quads + x / 4 + j / 4] : coef[a][at + j];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const float4 c0 = a == 0 ? c[j] : c[0], c1 = a == 0 ? c[j + 1] : c[1];
@@ -911,7 +915,8 @@ __device__ __forceinline__ void layer_quad(const Tables &g, const Fields<T> &f, 
     if (!(d.w & 15u)) return;  // (it only keeps a face for the quads above)
     LayerState<T> s;
     load_layer(f.cell_old, g.layer_lanes, q, d, s);
-    step_layer<T, SCALED, COMP, STREAM>(g, f, g.layer_coef, q, d, s);
+    const float4 *const coef[3] = {g.layer_coef_x, g.layer_coef[1], g.layer_coef[2]};
+    step_layer<T, SCALED, COMP, STREAM>(g, f, coef, q, d, s);
     store_layer<STREAM>(f.cell_new, g.layer_lanes, q, d, s);
 }
 

@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(kResidentThreads<T, WIDE, LAYER>, 1)
         float4 *at = reinterpret_cast<float4 *>(smem);
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            for (uint32_t x = threadIdx.x; x < p.coefs[a]; x += kThreads) at[x] = g.layer_coef[a][x];
+            for (uint32_t x = threadIdx.x; x < p.coefs[a]; x += kThreads) at[x] = (a == 0 ? g.layer_coef_x : g.layer_coef[a])[x];
             coef[a] = at, at += p.coefs[a];
         }
         for (uint32_t t = warp; t < layer; t += kWarps) {
