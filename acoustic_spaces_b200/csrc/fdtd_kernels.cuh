@@ -633,6 +633,11 @@ __device__ __forceinline__ RowEntry row_entry(const Tables &g, uint32_t k) {
 
 constexpr int kPackedLinks = 12;  // the directions a RowEntry holds
 
+// A fitted row has 3 to 8 links, few of them more (the source's have 18): a warp whose rows all have no
+// more than this issues that many slots' instructions in place of eighteen.
+constexpr int kFewLinks = 8;
+__device__ __forceinline__ bool more_links(uint32_t links) { return __any_sync(__activemask(), links > (uint32_t)kFewLinks); }
+
 // (offset: the directions' steps in the pitched grid, in shared memory: lanes index it apart.)
 template <typename T, int SLOTS, bool COMP, bool STREAM = true>
 __device__ __forceinline__ void special_row(const Tables &g, const Fields<T> &f, const uint32_t k, const RowEntry &e,
@@ -731,7 +736,10 @@ __global__ void __launch_bounds__(kBlock) special_kernel(const Tables g, const F
     for (; k < K; k += step) {
         const RowEntry e = next;
         if (k + step < K) next = row_entry<SLOTS, true>(g, k + step);
-        special_row<T, SLOTS, COMP>(g, f, k, e, offset);
+        if (SLOTS > kFewLinks && !more_links(e.links))
+            special_row<T, kFewLinks, COMP>(g, f, k, e, offset);
+        else
+            special_row<T, SLOTS, COMP>(g, f, k, e, offset);
     }
 }
 

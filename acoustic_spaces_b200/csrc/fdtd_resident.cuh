@@ -451,8 +451,8 @@ __global__ void __launch_bounds__(kResidentThreads<T, WIDE, LAYER>, 1)
                 if (p.staged) {
                     if (g.link_mask)
                         staged_row<T, 0, COMP>(g, m, f, r - r0, cur, r, s0);
-                    else if (g.link_slots <= 6)
-                        staged_row<T, 6, COMP>(g, m, f, r - r0, cur, r, s0);
+                    else if (!more_links(m.link_at[r - r0 + 1] - m.link_at[r - r0]))
+                        staged_row<T, kFewLinks, COMP>(g, m, f, r - r0, cur, r, s0);
                     else
                         staged_row<T, 18, COMP>(g, m, f, r - r0, cur, r, s0);
                 } else {
