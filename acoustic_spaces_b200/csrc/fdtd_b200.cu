@@ -26,6 +26,7 @@
 #include "fdtd_adjoint.cuh"
 #include "fdtd_b200.h"
 #include "fdtd_flow.cuh"
+#include "fdtd_columns.cuh"
 #include "fdtd_kernels.cuh"
 #include "fdtd_resident.cuh"
 #include "fdtd_resident_adjoint.cuh"
@@ -84,6 +85,9 @@ struct AdjointState {
     bool resident = false, clustered = false;
     const uint2 *columns = nullptr;
     uint32_t column_count = 0, blocks = 0, cells_at = 0, smem = 0;
+    // The launched reverse sweep's columns (null: bulk_kernel's tiles).
+    const uint2 *sweep_columns = nullptr;
+    uint32_t sweep_count = 0;
 };
 
 }  // namespace
@@ -165,6 +169,9 @@ struct fdtd_solver {
     uint32_t resident_keep_layer = 0, resident_rows_at = 0, resident_layer_at = 0;
     const uint32_t *link_start = nullptr;
     const uint2 *row_links = nullptr;
+    // The launched sweep's columns (null: bulk_kernel's tiles, as fdtd_set_tiles has chosen).
+    const uint2 *sweep_columns = nullptr;
+    uint32_t sweep_count = 0;
     void *resident_work = nullptr;  // the layer's state of the tasks that shared memory does not hold
     std::vector<uint32_t> host_state_start;
     unsigned int *arrived = nullptr;
@@ -507,6 +514,42 @@ int tensor_map(fdtd_solver *s, CUtensorMap *map, void *base, CUtensorMapDataType
     return FDTD_OK;
 }
 
+// The columns of quads of the interior, `planes` planes at most each: every run of planes that
+// holds interior cells, from its first, so that a column's first plane holds one.
+void interior_columns(const fdtd_solver *s, const std::vector<uint8_t> &types, uint64_t planes, std::vector<uint2> &columns) {
+    columns.clear();
+    const BulkArgs &bk = s->bulk;
+    if (!s->interior || types.empty()) return;
+    const uint64_t quads = s->pitch / 4, plane = s->pitch * s->ny;
+    std::vector<uint32_t> masks(quads);
+    for (uint64_t z0 = bk.z0; z0 < bk.z1; z0 += planes)
+        for (uint64_t y = bk.y0; y < bk.y1; ++y) {
+            std::fill(masks.begin(), masks.end(), 0u);
+            for (uint64_t z = z0, end = std::min<uint64_t>(z0 + planes, bk.z1); z < end; ++z) {
+                const uint8_t *row = &types[plane * z + s->pitch * y];
+                for (uint64_t q = 0; q < quads; ++q) {
+                    uint32_t four;
+                    std::memcpy(&four, row + 4 * q, 4);
+                    if (!four) continue;
+                    uint32_t mask = 0;
+                    for (int j = 0; j < 4; ++j) mask |= (((four >> (8 * j)) & 255u) == kInterior ? 1u : 0u) << j;
+                    masks[q] |= mask << (4 * (z - z0));
+                }
+            }
+            for (uint64_t q = 0; q < quads; ++q) {
+                if (!masks[q]) continue;
+                const int skip = __builtin_ctz(masks[q]) / 4;
+                columns.push_back(make_uint2((uint32_t)(plane * (z0 + skip) + s->pitch * y + 4 * q), masks[q] >> (4 * skip)));
+            }
+        }
+}
+
+// Planes a column of the launched sweep spans at most: a longer one reads the planes beyond its ends for
+// more cells, a shorter one keeps more blocks' loads in flight. Measured, 2, 4 and 8 planes: the 16M-cell box with a
+// speed field 50.8, 50.6 and 51.8 us a step, the batch of boxes 47.5, 46.0 and 46.7, outdoors 80.3, 79.4 and 84.6; the
+// wide stencil, whose columns keep nine rows in registers, 41.5, 35.8 and 33.3 on 9.7M cells.
+uint64_t sweep_planes(const fdtd_solver *s) { return s->wide ? 8 : 4; }
+
 // Planes a tile by default: at most 64, halved while there would be fewer than 8 tiles a
 // multiprocessor (at least 8 planes).
 uint64_t default_chunk(const fdtd_solver *s) {
@@ -677,6 +720,24 @@ int set_up_kernels(fdtd_solver *s) {
     return FDTD_OK;
 }
 
+template <typename T>
+SweepArgs<T> sweep_args(const fdtd_solver *s, const uint2 *columns, uint32_t count) {
+    SweepArgs<T> p{};
+    p.columns = columns, p.count = count;
+    p.pitch = s->tables.pitch, p.plane = s->tables.plane;
+    p.scale = s->scale_device;
+    p.d = static_cast<T *>(s->increment);
+    p.axial = s->bulk.axial, p.diagonal = s->bulk.diagonal, p.centre = s->bulk.centre, p.total = s->bulk.total;
+    p.residual = s->bulk.residual;
+    return p;
+}
+
+template <typename T, bool WIDE, bool SCALED, bool COMP>
+void launch_columns(const fdtd_solver *s, const uint2 *columns, uint32_t count, const T *b, T *a) {
+    column_kernel<T, WIDE, SCALED, COMP><<<(count + kColumnThreads - 1) / kColumnThreads, kColumnThreads, 0, s->stream>>>(
+        sweep_args<T>(s, columns, count), b, a);
+}
+
 // One launch of the sweep in the handle's shape.
 template <typename T, bool WIDE, bool SCALED, bool COMP>
 void launch_bulk(const fdtd_solver *s, const CUtensorMap &mb, const CUtensorMap &ma, const BulkArgs &args) {
@@ -824,7 +885,10 @@ int launch_piece(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
             args.d = f.d;
             const int cur = flip ? 0 : 1, prev = flip ? 1 : 0;
             // (Compensated: the increments stand in the previous pressure's place.)
-            launch_bulk<T, WIDE, SCALED, COMP>(s, s->map_b[cur], COMP ? s->map_d : s->map_a[prev], args);
+            if (s->sweep_columns)
+                launch_columns<T, WIDE, SCALED, COMP>(s, s->sweep_columns, s->sweep_count, f.b, f.a);
+            else
+                launch_bulk<T, WIDE, SCALED, COMP>(s, s->map_b[cur], COMP ? s->map_d : s->map_a[prev], args);
         }
         if (ev) CUDA_TRY(s, cudaEventRecord(ev[1], s->stream));
         if (ev) CUDA_TRY(s, cudaEventRecord(ev[2], layer));
@@ -954,10 +1018,7 @@ int launch_resident(fdtd_solver *s, const float *d_signal, uint64_t steps, doubl
             a.layer[k] = static_cast<T *>(s->layer_state[from]);
         }
         a.d = static_cast<T *>(s->increment);
-        a.scale = s->scale_device;
-        a.columns = s->columns, a.column_count = s->column_count;
-        a.axial = s->bulk.axial, a.diagonal = s->bulk.diagonal, a.centre = s->bulk.centre, a.total = s->bulk.total;
-        a.residual = s->bulk.residual;
+        a.air = sweep_args<T>(s, s->columns, s->column_count);
         a.signal = d_signal + done;
         a.link_start = s->link_start, a.links = s->row_links, a.staged = s->resident_staged ? 1 : 0;
         a.keep_layer = s->resident_keep_layer, a.rows_at = s->resident_rows_at, a.layer_at = s->resident_layer_at;
@@ -994,36 +1055,6 @@ int dispatch_run(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
     return launch_steps<T, W, S, C>(s, d_signal, steps, d_out, stride);
 }
 
-// The columns of quads of the interior, `planes` planes at most each: every run of planes that
-// holds interior cells, from its first, so that a column's first plane holds one.
-void interior_columns(const fdtd_solver *s, const std::vector<uint8_t> &types, uint64_t planes, std::vector<uint2> &columns) {
-    columns.clear();
-    const BulkArgs &bk = s->bulk;
-    if (!s->interior || types.empty()) return;
-    const uint64_t quads = s->pitch / 4, plane = s->pitch * s->ny;
-    std::vector<uint32_t> masks(quads);
-    for (uint64_t z0 = bk.z0; z0 < bk.z1; z0 += planes)
-        for (uint64_t y = bk.y0; y < bk.y1; ++y) {
-            std::fill(masks.begin(), masks.end(), 0u);
-            for (uint64_t z = z0, end = std::min<uint64_t>(z0 + planes, bk.z1); z < end; ++z) {
-                const uint8_t *row = &types[plane * z + s->pitch * y];
-                for (uint64_t q = 0; q < quads; ++q) {
-                    uint32_t four;
-                    std::memcpy(&four, row + 4 * q, 4);
-                    if (!four) continue;
-                    uint32_t mask = 0;
-                    for (int j = 0; j < 4; ++j) mask |= (((four >> (8 * j)) & 255u) == kInterior ? 1u : 0u) << j;
-                    masks[q] |= mask << (4 * (z - z0));
-                }
-            }
-            for (uint64_t q = 0; q < quads; ++q) {
-                if (!masks[q]) continue;
-                const int skip = __builtin_ctz(masks[q]) / 4;
-                columns.push_back(make_uint2((uint32_t)(plane * (z0 + skip) + s->pitch * y + 4 * q), masks[q] >> (4 * skip)));
-            }
-        }
-}
-
 // The columns with as many planes each as leave every warp one task (a step is then one chain of
 // loads); where the tasks (`other` ones beside the columns') are more than the warps, the choice of the
 // fewest planes in turn a warp, two planes counted for a column's first loads. (Measured, 1, 2, 3, 4, 6 and 8
@@ -1043,22 +1074,21 @@ void choose_columns(const fdtd_solver *s, const std::vector<uint8_t> &types, uin
     if (best > 1) interior_columns(s, types, best, columns);
 }
 
-// Whether the grid takes the resident stepper: the bytes that its steps touch, against a limit.
-// Below it they stay in L2 and a step costs its barrier, not its launches; beyond it the launched
-// steps' pipelined sweep keeps more of the DRAM's bandwidth. Measured, us a step, launched and
-// resident: FP32 boxes of 6.3M cells (50 MB) 20.5 and 16.1-18.2, 11.5M (92 MB) 39-49 and 34.6-36.4, 16M (128
-// MB) 50.3 and 49.0, 21M 62.8 and 76; compensated 6.3M (75 MB) 25.7 and 20.5, 11.5M (138 MB) 48 and 53-58; with a
-// matched layer FP32 3M (0.9M layer cells, 74 MB) 28.7 and 25.6, 5.9M (131 MB) 39 and 56; the wide
-// stencil 9.7M (78 MB) 73.6 and 69.5. In double the launched sweep is the slower one and a plain box
-// still gains at 184 MB (65.8 and 59.8; at 255 MB 85.9 and 90.4), the wide stencil not beyond 61 MB (51.4
-// and 51.5 there).
+// Whether the grid takes the resident stepper, by the bytes that its steps touch. It saves a step's
+// launches and event waits; the launched kernels, lean ones of many blocks, keep more loads in flight.
+// Measured, us a step, launched (each kind on its stream) and resident, at so many air cells:
+//   FP32 boxes 0.58M 6.1 and 4.2, 1.5M 7.0 and 6.5, 2.6M 7.5 and 9.0, 8.6M 21.5 and 25.0; compensated 1.5M 7.4 and 7.3, 2.6M 8.7
+//   and 10.4; the wide stencil 0.86M 8.1 and 6.5, 1.7M 9.5 and 9.4, 3.5M 13.8 and 16.8;
+//   FP32 with a matched layer 0.34M (0.19M layer cells) 6.9 and 4.9, 0.68M 8.2 and 8.1, 1.3M 13.1 and 14.0-17.2;
+//   double 1.5M 10.9 and 9.8, 2.6M 14.1 and 14.5, 4.3M 23.8 and 22.4, 8.6M 48.0 and 45.3, 10.8M 58.6 and 61.3; with a layer
+//   0.68M 12.6 and 11.5, 1.3M 24.6 and 20.2-23.3, 2.1M 37-44 and 36-45; wide 0.86M 10.9 and 10.5, 1.7M 14.6 and 16.1.
 bool takes_resident(const fdtd_solver *s, const fdtd_layout *L) {
     if (L->flow_count) return false;
     const uint64_t e = s->precision == FDTD_FP64 ? 8 : 4, MB = 1000 * 1000;
-    const uint64_t a_cell = 2 * e + (s->precision == FDTD_FP32_COMPENSATED ? e : 0) + (s->scaled ? 4 : 0);
+    const uint64_t a_cell = 2 * e + (s->precision == FDTD_FP32_COMPENSATED ? e : 0);
     const uint64_t touched = a_cell * s->air + 2 * kLayerSlots * e * L->layer_count;
-    if (e == 4) return touched <= 100 * MB;
-    return touched <= (s->wide ? 50 * MB : (L->layer_count ? 80 * MB : 190 * MB));
+    if (L->layer_count) return touched <= (e == 4 ? 30 : 72) * MB;
+    return e == 4 || s->wide ? touched <= a_cell * 1600000 && touched <= 20 * MB : touched <= 140 * MB;
 }
 
 // The resident stepper's launch and lists for the grid, once takes_resident has said yes.
@@ -1349,6 +1379,10 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
         s->plain_count = (uint32_t)plain.size();
         if ((rc = set_up(s))) return rc;
         if ((rc = use_shape(s, 0, s->bulk_chunk))) return rc;
+        std::vector<uint2> columns;
+        interior_columns(s, s->host_types, sweep_planes(s), columns);
+        if ((rc = upload(s, columns.data(), columns.size(), &s->sweep_columns))) return rc;
+        s->sweep_count = (uint32_t)columns.size();
     }
 
     // Special rows with 32-bit pitched indices.
@@ -1998,6 +2032,12 @@ int set_up_adjoint(fdtd_solver *s) {
     if ((rc = adjoint_lists(s, lists))) return rc;
     Owned owned{s};
     if ((rc = place_adjoint(s, lists, owned, s->adjoint))) return rc;
+    if (s->sweep_columns) {
+        std::vector<uint2> columns;
+        interior_columns(s, lists.types, sweep_planes(s), columns);
+        if ((rc = upload(s, columns.data(), columns.size(), &s->adjoint.sweep_columns))) return rc;
+        s->adjoint.sweep_count = (uint32_t)columns.size();
+    }
     if (s->resident) {
 #define SET_F(W, S, L) set_up_reverse<float, W, S, L>(s, lists)
 #define SET_D(W, S, L) set_up_reverse<double, W, S, L>(s, lists)
@@ -2257,11 +2297,7 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
     auto reverse_resident = [&](uint64_t first, uint64_t count, const T *u, const T *w, const double *d, uint64_t stride) -> int {
         ReverseArgs<T> a{};
         a.t = t;
-        a.sweep.g.pitch = s->tables.pitch, a.sweep.g.plane = s->tables.plane;
-        a.sweep.scale = s->scale_device;
-        a.sweep.columns = adj.columns, a.sweep.column_count = adj.column_count;
-        a.sweep.axial = s->bulk.axial, a.sweep.diagonal = s->bulk.diagonal;
-        a.sweep.centre = s->bulk.centre, a.sweep.total = s->bulk.total;
+        a.sweep = sweep_args<T>(s, adj.columns, adj.column_count);
         for (int k = 0; k < 2; ++k) {
             const int from = k ? 1 - x : x;
             a.lam[k] = static_cast<T *>(adj.lam[from]), a.om[k] = static_cast<T *>(adj.om[from]);
@@ -2341,7 +2377,14 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
                 CUDA_TRY(s, cudaEventRecord(s->joined[2], s->layer_stream));
             }
             CUDA_TRY(s, cudaEventRecord(s->joined[1], s->side));
-            if (s->bulk_blocks) {
+            if (adj.sweep_columns) {
+#define SWEEP(W, S) launch_columns<T, W, S, false>(s, adj.sweep_columns, adj.sweep_count, lam_next, lam_out)
+                if (s->wide)
+                    s->scaled ? SWEEP(true, true) : SWEEP(true, false);
+                else
+                    s->scaled ? SWEEP(false, true) : SWEEP(false, false);
+#undef SWEEP
+            } else if (s->bulk_blocks) {
                 // The forward sweep of the grid's own kind (with a speed field it steps v = s lam).
                 BulkArgs args = s->bulk;
                 args.a = lam_out;
@@ -3141,10 +3184,13 @@ int fdtd_set_tiles(fdtd_solver *s, int shape, uint64_t planes) {
     if (planes < 1 || planes > 1024) return fail(s, FDTD_EINVAL, "planes a tile are 1 to 1024");
     if (!s->bulk_tiles) return FDTD_OK;  // no interior cells: no sweep
     if (s->shape_per_sm[shape] < 1) return fail(s, FDTD_EINVAL, "the tile shape does not fit a multiprocessor here");
+    // (What fdtd_get_tiles reports of a grid that sweeps by columns, given back, leaves it so.)
+    if (s->sweep_columns && shape == s->bulk_shape && planes == s->bulk_chunk) return FDTD_OK;
     DeviceGuard guard(s->device);
     for (cudaStream_t stream : {s->stream, s->side, s->layer_stream}) CUDA_TRY(s, cudaStreamSynchronize(stream));
     Kept{s}.drop_graphs();
     s->resident = false;
+    s->sweep_columns = nullptr;  // (the list stays with the handle's allocations)
     return use_shape(s, shape, planes);
 }
 
@@ -3254,7 +3300,7 @@ int fdtd_autotune(fdtd_solver *s, uint64_t trial_steps, int *layer_per_sm, int *
     // streams beside one another or in turn, the layer's and the special rows' blocks an SM) given
     // the tiles; then the tiles once more given the launches, as the kernels share the SMs.
     auto tune_tiles = [&]() -> int {
-        if (!s->bulk_tiles) return FDTD_OK;
+        if (!s->bulk_tiles || s->sweep_columns) return FDTD_OK;
         const uint64_t base = default_chunk(s);
         float best_tiles = -1.0f;
         int best_shape = s->bulk_shape, r = FDTD_OK;

@@ -40,8 +40,11 @@ constexpr int kLayerSlots = 6;
 // ---- the bulk sweep's tiles ------------------------------------------------------------------
 constexpr int kHX = 4;                          // x halo of the pressure tile: 16 bytes of floats
 constexpr uint32_t kSpinLimit = 1u << 24;       // bounded waits: then the block gives up
-constexpr int kLayerPerSm = 8;                  // blocks an SM of the matched-layer kernel
-constexpr int kSpecialPerSm = 4;                // blocks an SM of the special rows' kernel
+// Blocks an SM of the matched-layer and special-row kernels (0: a thread a row) before fdtd_autotune has
+// chosen: beside the sweep by columns, 4 and 0 took 13.1 us a step on the 1.3M-cell auditorium and 29.1 on 4M cells
+// with a layer, 8 and 4 14.0 and 32.3; 21.5 against 23.7 on an 8.6M-cell box.
+constexpr int kLayerPerSm = 4;
+constexpr int kSpecialPerSm = 0;
 
 // A tile shape of the bulk sweep: TX x TY cells a plane, a ring of STAGES plane stages (the three
 // in use and STAGES - 3 loaded ahead), THREADS threads a block. Each thread updates ROWS rows of

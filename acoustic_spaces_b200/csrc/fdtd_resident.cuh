@@ -10,23 +10,16 @@
 // in their order: the results are equal to the bit.
 #pragma once
 
-#include "fdtd_kernels.cuh"
+#include "fdtd_columns.cuh"
 
 namespace fdtd {
-
-constexpr int kColumnPlanes = 8;  // planes an item of the interior's list spans at most (4 bits each)
 
 template <typename T>
 struct ResidentArgs {
     Tables g;
     T *u[2], *w[2], *layer[2];  // [1]: the current ones at the launch's start
     T *d;                       // COMP: the increments
-    const float *scale;         // with a speed field: each pitched cell's scale
-    // The interior air: columns of quads along z, {the first quad's pitched index, the interior
-    // cells of each plane, four bits a plane from the lowest}.
-    const uint2 *columns;
-    uint32_t column_count;
-    float axial, diagonal, centre, total, residual;
+    SweepArgs<T> air;           // the interior air's columns
     const float *signal;  // the drive of the launch's first step
     // The special rows' links row by row (their starts, then {weight, offset} each), and whether each
     // block keeps its rows' tables and branch velocities in shared memory over the steps.
@@ -75,152 +68,6 @@ __device__ __forceinline__ bool step_barrier(unsigned int *arrived, unsigned int
         if (failed) atomicOr(error, 1u);
     }
     return !__syncthreads_or(failed);
-}
-
-// ---- the interior air ----------------------------------------------------------------------------
-
-// A quad's new pressures (fdtd.hpp:242-288) from its own pressures h, its neighbours before and
-// after along x (left, right the cells beside the quad), y and z, and with the wide stencil the
-// twelve edge sums; pv the previous pressures (COMP: the increments).
-template <typename T, bool WIDE, bool SCALED, bool COMP>
-struct Update {
-    T axial, diagonal, centre, total, residual;
-    template <class Edges>
-    __device__ __forceinline__ void operator()(const Quad<T> &h, T left, T right, const Quad<T> &ym, const Quad<T> &yp,
-                                               const Quad<T> &zm, const Quad<T> &zp, const Quad<T> &pv, const Quad<T> &sc,
-                                               Edges edges, Quad<T> &next, Quad<T> &step) const {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const T here = h.v[j];
-            const T xm = j == 0 ? left : h.v[j - 1], xp = j == 3 ? right : h.v[j + 1];
-            if (COMP) {
-                const T sum = (xm - here) + (xp - here) + (ym.v[j] - here) + (yp.v[j] - here) + (zm.v[j] - here) +
-                              (zp.v[j] - here);
-                const T around = WIDE ? edges(j, here) : (T)0;
-                T s;
-                if (SCALED) {
-                    s = WIDE ? pv.v[j] + (sc.v[j] * axial) * sum + (sc.v[j] * diagonal) * around + (sc.v[j] * residual) * here
-                             : pv.v[j] + (sc.v[j] * axial) * sum + (sc.v[j] * residual) * here;
-                } else {
-                    s = WIDE ? pv.v[j] + axial * sum + diagonal * around + residual * here
-                             : pv.v[j] + axial * sum + residual * here;
-                }
-                next.v[j] = here + s;
-                step.v[j] = s;
-                continue;
-            }
-            const T sum = xm + xp + ym.v[j] + yp.v[j] + zm.v[j] + zp.v[j];
-            const T around = WIDE ? edges(j, (T)0) : (T)0;
-            if (SCALED) {
-                next.v[j] = WIDE ? ((T)2 - total * sc.v[j]) * here + (sc.v[j] * axial) * sum + (sc.v[j] * diagonal) * around - pv.v[j]
-                                 : ((T)2 - total * sc.v[j]) * here + (sc.v[j] * axial) * sum - pv.v[j];
-            } else {
-                next.v[j] = WIDE ? centre * here + axial * sum + diagonal * around - pv.v[j] : centre * here + axial * sum - pv.v[j];
-            }
-        }
-    }
-};
-
-// What a plane of a 7-point column loads beside the pressures it keeps from the plane before: the
-// pressures a plane on, a row before and after and beside the quad, and the previous pressures.
-template <typename T>
-struct PlaneLoads {
-    Quad<T> zp, ym, yp, pv;
-    T left, right;
-    __device__ __forceinline__ void load(const T *b, const T *before, uint32_t i, uint32_t pitch, uint32_t plane) {
-        zp = load_quad(b + i + plane);
-        ym = load_quad(b + i - pitch);
-        yp = load_quad(b + i + pitch);
-        pv = load_quad(before + i);
-        left = b[i - 1], right = b[i + 4];
-    }
-};
-
-// A column of quads along z, the 7-point stencil: each plane's loads are issued while the plane
-// before is worked out, and a quad's pressures serve the planes before and after it from registers.
-// (The cells beside a quad by shuffles from the lanes beside, in place of scalar loads, made a step of
-// 2.9M cells 12.6 us in place of 9.0: the lanes' loads then wait for one another.)
-template <typename T, bool SCALED, bool COMP>
-__device__ __forceinline__ void step_column(const ResidentArgs<T> &p, const T *b, T *a, uint2 column) {
-    const uint32_t pitch = p.g.pitch, plane = p.g.plane;
-    const T *before = COMP ? p.d : a;
-    const Update<T, false, SCALED, COMP> update{(T)p.axial, (T)p.diagonal, (T)p.centre, (T)p.total, (T)p.residual};
-    uint32_t i = column.x, masks = column.y;
-    Quad<T> zm = load_quad(b + i - plane), h = load_quad(b + i);
-    PlaneLoads<T> now, then;
-    now.load(b, before, i, pitch, plane);
-    for (;;) {
-        const uint32_t mask = masks & 15u;
-        masks >>= 4;
-        if (masks) then.load(b, before, i + plane, pitch, plane);
-        if (mask) {
-            Quad<T> next, step;
-            update(h, now.left, now.right, now.ym, now.yp, zm, now.zp, now.pv, scales<T, SCALED>(p.scale, i),
-                   [](int, T) { return (T)0; }, next, step);
-            store_cells<false>(a + i, next, mask);
-            if (COMP) store_cells<false>(p.d + i, step, mask);
-        }
-        if (!masks) return;
-        zm = h, h = now.zp, now = then;
-        i += plane;
-    }
-}
-
-// Six cells of a row: a quad and the cells beside it, where a column's interior cells need them (a
-// quad at the grid's first cells has no cell before it, and its first cell is on the edge).
-template <typename T>
-struct Row {
-    T v[6];
-    __device__ __forceinline__ void load(const T *p, bool left, bool right) {
-        const Quad<T> q = load_quad(p);
-        v[0] = left ? p[-1] : (T)0, v[5] = right ? p[4] : (T)0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v[1 + j] = q.v[j];
-    }
-    __device__ __forceinline__ Quad<T> quad() const { return {{v[1], v[2], v[3], v[4]}}; }
-};
-
-// The same with the 19-point stencil: three rows of six cells of each of three planes.
-template <typename T, bool SCALED, bool COMP>
-__device__ __forceinline__ void step_wide_column(const ResidentArgs<T> &p, const T *b, T *a, uint2 column) {
-    const uint32_t pitch = p.g.pitch, plane = p.g.plane;
-    const T *before = COMP ? p.d : a;
-    const Update<T, true, SCALED, COMP> update{(T)p.axial, (T)p.diagonal, (T)p.centre, (T)p.total, (T)p.residual};
-    uint32_t i = column.x, masks = column.y;
-    const bool left = (masks & 0x11111111u) != 0, right = (masks & 0x88888888u) != 0;
-    Row<T> z[3][3];  // [plane before, this, after][row before, this, after]
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-#pragma unroll
-        for (int r = 0; r < 3; ++r) z[k][r].load(b + i + (k - 1) * (int64_t)plane + (r - 1) * (int64_t)pitch, left, right);
-    while (masks) {
-        const uint32_t mask = masks & 15u;
-        masks >>= 4;
-#pragma unroll
-        for (int r = 0; r < 3; ++r) z[2][r].load(b + i + plane + (r - 1) * (int64_t)pitch, left, right);
-        if (mask) {
-            const Quad<T> pv = load_quad(before + i);
-            Quad<T> next, step;
-            update(
-                z[1][1].quad(), z[1][1].v[0], z[1][1].v[5], z[1][0].quad(), z[1][2].quad(), z[0][1].quad(), z[2][1].quad(),
-                pv, scales<T, SCALED>(p.scale, i),
-                [&](int j, T here) {
-                    const T *m = z[1][0].v + j, *q = z[1][2].v + j, *l = z[0][1].v + j, *h = z[2][1].v + j;
-                    if (COMP)
-                        return (m[0] - here) + (m[2] - here) + (q[0] - here) + (q[2] - here) + (l[0] - here) + (l[2] - here) +
-                               (h[0] - here) + (h[2] - here) + (z[0][0].v[j + 1] - here) + (z[0][2].v[j + 1] - here) +
-                               (z[2][0].v[j + 1] - here) + (z[2][2].v[j + 1] - here);
-                    return m[0] + m[2] + q[0] + q[2] + l[0] + l[2] + h[0] + h[2] + z[0][0].v[j + 1] + z[0][2].v[j + 1] +
-                           z[2][0].v[j + 1] + z[2][2].v[j + 1];
-                },
-                next, step);
-            store_cells<false>(a + i, next, mask);
-            if (COMP) store_cells<false>(p.d + i, step, mask);
-        }
-#pragma unroll
-        for (int r = 0; r < 3; ++r) z[0][r] = z[1][r], z[1][r] = z[2][r];
-        i += plane;
-    }
 }
 
 // ---- the special rows ------------------------------------------------------------------------------
@@ -358,7 +205,7 @@ __global__ void __launch_bounds__(kResidentThreads<T, WIDE, LAYER>, 1)
     };
     uint32_t rows0, layer0 = 0, reads0, air0;
     const uint32_t rows = share(g.specials, rows0), layer = LAYER ? share(g.layer_quads, layer0) : 0u;
-    const uint32_t reads = share(p.gathered_count, reads0), air = share(p.column_count, air0);
+    const uint32_t reads = share(p.gathered_count, reads0), air = share(p.air.count, air0);
     const uint32_t all = rows + layer + reads + air;
     // The rows staged in shared memory.
     const uint32_t r0 = min(rows0 * 32, g.specials), r1 = min((rows0 + rows) * 32, g.specials);
@@ -425,8 +272,8 @@ __global__ void __launch_bounds__(kResidentThreads<T, WIDE, LAYER>, 1)
             return e;
         }
         const uint32_t c = (air0 + t - reads) * 32 + lane;
-        if (c < p.column_count) {
-            const uint2 column = __ldg(p.columns + c);
+        if (c < p.air.count) {
+            const uint2 column = __ldg(p.air.columns + c);
             e.x = column.x, e.y = column.y;
         }
         return e;
@@ -474,9 +321,9 @@ __global__ void __launch_bounds__(kResidentThreads<T, WIDE, LAYER>, 1)
                 if (c < p.gathered_count) p.gathered[(uint64_t)k * p.gathered_count + c] = f.b[e.x];
             } else if (e.y) {
                 if constexpr (WIDE)
-                    step_wide_column<T, SCALED, COMP>(p, f.b, f.a, make_uint2(e.x, e.y));
+                    step_wide_column<T, SCALED, COMP>(p.air, f.b, f.a, make_uint2(e.x, e.y));
                 else
-                    step_column<T, SCALED, COMP>(p, f.b, f.a, make_uint2(e.x, e.y));
+                    step_column<T, SCALED, COMP>(p.air, f.b, f.a, make_uint2(e.x, e.y));
             }
         }
         if (k + 1 < p.steps && !step_barrier(p.arrived, (k + 1) * gridDim.x, p.clustered, p.error)) break;

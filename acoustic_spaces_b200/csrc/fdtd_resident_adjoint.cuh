@@ -13,7 +13,7 @@ namespace fdtd {
 template <typename T>
 struct ReverseArgs {
     AdjointTables t;
-    ResidentArgs<T> sweep;  // the interior sweep's columns, coefficients and strides
+    SweepArgs<T> sweep;
     // Each launch's first step reads lam[0] (the level after) and its companions and writes lam[1]; the
     // next the other way round.
     T *lam[2], *om[2], *tilde[2], *hat[2];
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kReverseThreads, 1) reverse_kernel(const __gri
     };
     uint32_t rows0, layer0 = 0, whole0, air0;
     const uint32_t rows = share(t.specials, rows0), layer = LAYER ? share(t.layers, layer0) : 0u;
-    const uint32_t whole = share(t.corrected, whole0), air = share(p.sweep.column_count, air0);
+    const uint32_t whole = share(t.corrected, whole0), air = share(p.sweep.count, air0);
     const uint32_t all = rows + layer + whole + air;
     // The stages.
     const uint32_t r0 = min(rows0 * 32, t.specials), r1 = min((rows0 + rows) * 32, t.specials);
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(kReverseThreads, 1) reverse_kernel(const __gri
                 layer_adjoint_cell<T>(t, c, lam_next, tilde, hat, lam_out, p.dloss, p.stride, step, next);
             } else {
                 const uint32_t c = (air0 + k - rows - whole - layer) * 32 + lane;
-                if (c < p.sweep.column_count) {
+                if (c < p.sweep.count) {
                     const uint2 column = __ldg(p.sweep.columns + c);
                     if constexpr (WIDE)
                         step_wide_column<T, SCALED, false>(p.sweep, lam_next, lam_out, column);

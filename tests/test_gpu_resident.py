@@ -1,4 +1,4 @@
-"""The resident stepper and the matched layer by quads on the sizes where they can go wrong, against
+"""The resident stepper, the sweep by columns and the matched layer by quads on the sizes where they can go wrong, against
 the oracle to the bit (needs a B200): rows that end within a quad or fill the pitch, one column to
 many tasks a warp, a cluster or the whole GPU, runs longer than a launch, layers whose cells come in
 any order, the layer's state in shared memory or not, and handles stepped from two threads."""
@@ -30,8 +30,10 @@ def _box(shape, *, speed=None, branches=2, receivers=2, seed=3):
     return layouts.cell_face_layout(room, grid, points[0], points[1:], speed=speed, rate=rate).layout
 
 
-def _equal(layout, drive, cuts, precision, solver=None):
-    gpu, oracle = solver or B200WaveSolver(layout, precision=precision), OracleSolver(layout, precision)
+def _equal(layout, drive, cuts, precision, launched=False):
+    gpu, oracle = B200WaveSolver(layout, precision=precision), OracleSolver(layout, precision)
+    if launched:
+        gpu.set_streams(1)
     a = np.concatenate([gpu.run(drive[i:j]) for i, j in zip(cuts[:-1], cuts[1:])], axis=1)
     assert np.array_equal(a, oracle.run(drive))
     mine, theirs = gpu.state(), oracle.state()
@@ -48,9 +50,10 @@ def _drive(steps, seed=0):
     "shape, speed",
     [((12, 9, 11), None), ((13, 16, 13), 0.9), ((28, 12, 14), None), ((60, 61, 10), None), ((77, 50, 47), 0.97), ((140, 90, 61), None)],
 )  # (12 + 4 cells fill the pitch of 16; 13 and 77 end within a quad; the last spans several tasks a warp)
-def test_gpu_boxes_of_odd_sizes_step_as_the_oracle_does(shape, speed, precision):
+@pytest.mark.parametrize("launched", [False, True])
+def test_gpu_boxes_of_odd_sizes_step_as_the_oracle_does(shape, speed, precision, launched):
     steps = 90 if np.prod(shape) < 1e5 else 40
-    _equal(_box(shape, speed=speed), _drive(steps), [0, 1, 34, steps], precision)
+    _equal(_box(shape, speed=speed), _drive(steps), [0, 1, 34, steps], precision, launched)
 
 
 def test_gpu_runs_longer_than_a_launch():
@@ -58,18 +61,19 @@ def test_gpu_runs_longer_than_a_launch():
 
 
 @pytest.mark.parametrize("precision", ["fp32", "fp64", "fp32c"])
-@pytest.mark.parametrize("count", [2, 9])
-def test_gpu_wide_grids_step_as_the_oracle_does(count, precision):
+@pytest.mark.parametrize("count, launched", [(2, False), (9, False), (9, True)])
+def test_gpu_wide_grids_step_as_the_oracle_does(count, launched, precision):
     layout, signal, _ = load_golden("resonant19")
     stacked = layouts.stack([layout] * count, across=3).layout
-    _equal(stacked, signal[:70], [0, 33, 70], precision)
+    _equal(stacked, signal[:70], [0, 33, 70], precision, launched)
 
 
 @pytest.mark.parametrize("precision", ["fp32", "fp64", "fp32c"])
-@pytest.mark.parametrize("cell", [0.3, 0.21, 0.16, 0.13])  # (0.13: more state than shared memory holds)
-def test_gpu_layers_step_as_the_oracle_does(cell, precision):
+@pytest.mark.parametrize("cell", [0.3, 0.21, 0.16, 0.13])  # (0.13: in double more state than shared memory holds)
+@pytest.mark.parametrize("launched", [False, True])
+def test_gpu_layers_step_as_the_oracle_does(cell, precision, launched):
     w = layouts.polyhedral_room(2, cell=cell, receivers=3, steps=1)
-    _equal(w.built.layout, _drive(45), [0, 20, 45], precision)
+    _equal(w.built.layout, _drive(45), [0, 20, 45], precision, launched)
 
 
 @pytest.mark.parametrize("name", ["open_layer", "open_layer_speed", "fitted_open"])
