@@ -64,8 +64,8 @@ struct AdjointTables {
     const double *read_weight;
     // The matched layer (fdtd.hpp:2242-2264): its cells (pitched), the packed per-axis tables
     // {keep, push, keep_face, push_face} by grid coordinate, each cell's scale with a speed field.
-    uint32_t layers;
-    const uint32_t *layer_cells;
+    uint32_t layers, lanes;
+    const uint32_t *layer_cells, *cell_lane;  // (each cell's lane among the forward's quads)
     const float4 *layer_coef[3];
     const float *layer_scale;
     uint32_t pitch, plane;
@@ -223,7 +223,7 @@ __device__ __forceinline__ void special_adjoint_row(const AdjointTables &t, uint
 //   dkf[x] += L^ lo,  dpf[x] -= L^ (b_i - b_(i-st)).
 
 // The six factors per axis a layer cell records per forward step, at factor f of cell c:
-// traj[f * layers + c]: q, hi' - lo', hi, b_(i+st) - b_i, lo, b_i - b_(i-st) for axis 0, then 1, 2.
+// traj[f * lanes + its lane]: q, hi' - lo', hi, b_(i+st) - b_i, lo, b_i - b_(i-st) for axis 0, then 1, 2.
 constexpr int kLayerFactors = 18;
 
 // The carried values (9 per cell, together: Q^' x3, L^' x3, H^' x3 at carried[kCarried c + v]) are
@@ -294,14 +294,15 @@ __device__ __forceinline__ void layer_hat_cell(const AdjointTables &t, uint32_t 
         hv[2 * a] = (T)c0.w * lo_hat;
         hv[2 * a + 1] = (T)c1.w * hi_hat;
         if (g && traj) {
-            const T *f = traj + (uint64_t)(6 * a) * L + c;
+            const uint64_t M = t.lanes;
+            const T *f = traj + (uint64_t)(6 * a) * M + t.cell_lane[c];
             double *gg = g + (uint64_t)(6 * a) * L + c;
             gg[0] += (double)q_hat * (double)f[0];
-            gg[(uint64_t)1 * L] += -(double)q_hat * (double)s * (double)f[(uint64_t)1 * L];
-            gg[(uint64_t)2 * L] += (double)hi_hat * (double)f[(uint64_t)2 * L];
-            gg[(uint64_t)3 * L] += -(double)hi_hat * (double)f[(uint64_t)3 * L];
-            gg[(uint64_t)4 * L] += (double)lo_hat * (double)f[(uint64_t)4 * L];
-            gg[(uint64_t)5 * L] += -(double)lo_hat * (double)f[(uint64_t)5 * L];
+            gg[(uint64_t)1 * L] += -(double)q_hat * (double)s * (double)f[1 * M];
+            gg[(uint64_t)2 * L] += (double)hi_hat * (double)f[2 * M];
+            gg[(uint64_t)3 * L] += -(double)hi_hat * (double)f[3 * M];
+            gg[(uint64_t)4 * L] += (double)lo_hat * (double)f[4 * M];
+            gg[(uint64_t)5 * L] += -(double)lo_hat * (double)f[5 * M];
         } else if (pending) {
             pending[(uint64_t)(3 * a) * L + c] = q_hat;
             pending[(uint64_t)(3 * a + 1) * L + c] = lo_hat;
@@ -330,7 +331,8 @@ __device__ __forceinline__ void layer_hat_cell(const AdjointTables &t, uint32_t 
 // The tables' products of `steps` steps whose Q^, L^, H^ waited (layer_hat_cell; step k's at waiting + 9 k
 // layers), with their forward factors: `traj` the first's, each next one's a step's factors before. The
 // steps' products are added in turn, one read and write of a cell's eighteen double sums for all of
-// them (their 288 bytes a cell are most of what a step of the tables' gradient moves).
+// them (their 288 bytes a cell are most of what a step of the tables' gradient moves). A row of blocks an
+// axis.
 template <typename T>
 __global__ void __launch_bounds__(kBlock) layer_pending_kernel(const AdjointTables t, const T *waiting, uint32_t steps,
                                                                const T *traj, double *g) {
@@ -338,27 +340,26 @@ __global__ void __launch_bounds__(kBlock) layer_pending_kernel(const AdjointTabl
     const uint32_t L = t.layers;
     if (c >= L) return;
     const T s = t.layer_scale ? (T)t.layer_scale[c] : (T)1;
+    const uint32_t a = blockIdx.y, lane = t.cell_lane[c];
+    const uint64_t M = t.lanes;
+    double *gg = g + (uint64_t)(6 * a) * L + c;
+    double sum[6];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        double *gg = g + (uint64_t)(6 * a) * L + c;
-        double sum[6];
-#pragma unroll
-        for (int f = 0; f < 6; ++f) sum[f] = gg[(uint64_t)f * L];
-#pragma unroll 2
-        for (uint32_t k = 0; k < steps; ++k) {
-            const T *w = waiting + (uint64_t)k * 9 * L + c;
-            const T *f = traj - (uint64_t)k * kLayerFactors * L + (uint64_t)(6 * a) * L + c;
-            const T q_hat = w[(uint64_t)(3 * a) * L], lo_hat = w[(uint64_t)(3 * a + 1) * L], hi_hat = w[(uint64_t)(3 * a + 2) * L];
-            sum[0] += (double)q_hat * (double)f[0];
-            sum[1] += -(double)q_hat * (double)s * (double)f[(uint64_t)1 * L];
-            sum[2] += (double)hi_hat * (double)f[(uint64_t)2 * L];
-            sum[3] += -(double)hi_hat * (double)f[(uint64_t)3 * L];
-            sum[4] += (double)lo_hat * (double)f[(uint64_t)4 * L];
-            sum[5] += -(double)lo_hat * (double)f[(uint64_t)5 * L];
-        }
-#pragma unroll
-        for (int f = 0; f < 6; ++f) gg[(uint64_t)f * L] = sum[f];
+    for (int f = 0; f < 6; ++f) sum[f] = gg[(uint64_t)f * L];
+#pragma unroll 4
+    for (uint32_t k = 0; k < steps; ++k) {
+        const T *w = waiting + ((uint64_t)k * 9 + 3 * a) * L + c;
+        const T *f = traj - (uint64_t)k * kLayerFactors * M + (uint64_t)(6 * a) * M + lane;
+        const T q_hat = w[0], lo_hat = w[(uint64_t)L], hi_hat = w[2 * (uint64_t)L];
+        sum[0] += (double)q_hat * (double)f[0];
+        sum[1] += -(double)q_hat * (double)s * (double)f[1 * M];
+        sum[2] += (double)hi_hat * (double)f[2 * M];
+        sum[3] += -(double)hi_hat * (double)f[3 * M];
+        sum[4] += (double)lo_hat * (double)f[4 * M];
+        sum[5] += -(double)lo_hat * (double)f[5 * M];
     }
+#pragma unroll
+    for (int f = 0; f < 6; ++f) gg[(uint64_t)f * L] = sum[f];
 }
 
 // The tangent's products of a step whose Q^, L^, H^ waited in `pending`, once its factors are

@@ -846,7 +846,7 @@ int launch_piece(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
             f.traj_w = static_cast<T *>(s->record_w) + (k + s->record_offset) * s->states;
         }
         // The matched layer's factors of step k (the gradient's recomputation).
-        if (s->record_layer) f.traj_layer = static_cast<T *>(s->record_layer) + k * kLayerFactors * s->layers;
+        if (s->record_layer) f.traj_layer = static_cast<T *>(s->record_layer) + k * kLayerFactors * g.layer_lanes;
         // The factors of step k along the tables' tangent (a gradient's recomputation, or a taped run).
         if (s->record_tangent) f.traj_tangent = static_cast<T *>(s->record_tangent) + k * s->tangent_factors;
         if (fork) {
@@ -1029,7 +1029,7 @@ int launch_resident(fdtd_solver *s, const float *d_signal, uint64_t steps, doubl
             a.traj_u = static_cast<T *>(s->record_u) + (done + s->record_offset) * s->specials;
             a.traj_w = static_cast<T *>(s->record_w) + (done + s->record_offset) * s->states;
         }
-        if (s->record_layer) a.traj_layer = static_cast<T *>(s->record_layer) + done * kLayerFactors * s->layers;
+        if (s->record_layer) a.traj_layer = static_cast<T *>(s->record_layer) + done * kLayerFactors * s->tables.layer_lanes;
         if (s->record_tangent) a.traj_tangent = static_cast<T *>(s->record_tangent) + done * s->tangent_factors;
         a.states = (uint32_t)s->states, a.tangent_factors = (uint32_t)s->tangent_factors;
         a.steps = (uint32_t)count;
@@ -1533,6 +1533,7 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
         g.layer_quads = (uint32_t)quads.size(), g.layer_lanes = 4 * g.layer_quads;
         if ((rc = upload(s, quads.data(), quads.size(), &g.layer_quad))) return rc;
         if ((rc = upload(s, lane_cell.data(), lane_cell.size(), &g.lane_cell))) return rc;
+        if ((rc = upload(s, s->layer_lane.data(), s->layer_lane.size(), &g.cell_lane))) return rc;
         for (int k = 0; k < 2; ++k)
             if ((rc = zeros(s, e * kLayerSlots * g.layer_lanes, &s->layer_state[k]))) return rc;
         const uint64_t len[3] = {nx + 1, ny + 1, nz + 1};
@@ -1924,6 +1925,7 @@ int place_adjoint(fdtd_solver *s, const AdjointLists &l, Pool &pool, AdjointStat
     // and the hats (six pitched levels) are the adjoint's own.
     t.layers = (uint32_t)s->layers;
     t.layer_cells = g.layer_cells;
+    t.lanes = g.layer_lanes, t.cell_lane = g.cell_lane;
     for (int axis = 0; axis < 3; ++axis) t.layer_coef[axis] = g.layer_coef[axis];
     t.layer_scale = g.layer_scale;
     t.pitch = g.pitch, t.plane = g.plane;
@@ -2196,7 +2198,7 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
     }
     const uint64_t level_bytes = e * s->n_device, state_bytes = e * S;
     // The matched layer: its factors of each step of a segment, and its gradient's sums per cell.
-    const uint64_t Lc = s->layers;
+    const uint64_t Lc = s->layers, lanes = s->tables.layer_lanes;
     const bool tangent = Lc && s->tangent;  // along a tangent of the tables, in place of the tables
     const bool tables = Lc && s->gradient_tables && !tangent;
     T *traj_layer = nullptr, *waiting = nullptr;
@@ -2204,7 +2206,7 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
     double *g_layer = nullptr, *table_sums = nullptr;
     const uint64_t coords = s->nx + s->ny + s->nz;
     if (tables) {
-        if ((rc = scratch.take(e * kLayerFactors * Lc * segment, &p))) return rc;
+        if ((rc = scratch.take(e * kLayerFactors * lanes * segment, &p))) return rc;
         traj_layer = static_cast<T *>(p);
         if ((rc = scratch.take(sizeof(double) * kLayerFactors * Lc, &p))) return rc;
         g_layer = static_cast<double *>(p);
@@ -2325,8 +2327,8 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
             const int r = reverse_resident(first, n, traj_u, traj_w, seg_dloss, segment);
             if (r != FDTD_OK) return r;
             const uint64_t products = std::min(n, first);  // (step 0 has its factors in the segment before)
-            if (products) layer_pending_kernel<T><<<layer_blocks, kBlock, 0, s->stream>>>(
-                    t, waiting, (uint32_t)products, traj_layer + (first - 1) * kLayerFactors * Lc, g_layer);
+            if (products) layer_pending_kernel<T><<<dim3(layer_blocks, 3), kBlock, 0, s->stream>>>(
+                    t, waiting, (uint32_t)products, traj_layer + (first - 1) * kLayerFactors * lanes, g_layer);
             CUDA_TRY(s, cudaGetLastError());
             if (n & 1) x = 1 - x;
             done += n;
@@ -2355,7 +2357,7 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
             LayerNext<T> next{static_cast<T *>(adj.hat[1 - xx]), static_cast<T *>(adj.carried), nullptr, nullptr,
                               tables ? g_layer : nullptr};
             if (tables) {
-                if (m > 0) next.traj = traj_layer + (m - 1) * kLayerFactors * Lc;
+                if (m > 0) next.traj = traj_layer + (m - 1) * kLayerFactors * lanes;
                 else next.pending = static_cast<T *>(adj.pending);
             }
             if (tangent) {
@@ -2511,8 +2513,8 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
         // The layer's products of this segment's last step, whose Q^, L^, H^ the segment after
         // left waiting: its factors are recorded now.
         if (tables && k + 1 < segments) {
-            layer_pending_kernel<T><<<layer_blocks, kBlock, 0, s->stream>>>(
-                t, static_cast<const T *>(adj.pending), 1, traj_layer + (count - 1) * kLayerFactors * Lc, g_layer);
+            layer_pending_kernel<T><<<dim3(layer_blocks, 3), kBlock, 0, s->stream>>>(
+                t, static_cast<const T *>(adj.pending), 1, traj_layer + (count - 1) * kLayerFactors * lanes, g_layer);
             CUDA_TRY(s, cudaGetLastError());
         }
         if (tangent && k + 1 < segments) {
@@ -2643,7 +2645,7 @@ size_t pool_bytes(const fdtd_solver *s, const AdjointLists &l, uint64_t steps, u
     total += 2 * pool_round(8 * K) + 3 * pool_round(8 * S);
     if (Lc) total += pool_round(4 * l.by_coord.size()) + pool_round(4 * l.coord_start.size());
     if (Lc && s->gradient_tables && !s->tangent)
-        total += pool_round(e * kLayerFactors * Lc * segment) + pool_round(8 * kLayerFactors * Lc) +
+        total += pool_round(e * kLayerFactors * s->tables.layer_lanes * segment) + pool_round(8 * kLayerFactors * Lc) +
                  pool_round(8 * 6 * (s->nx + s->ny + s->nz));
     if (Lc && s->tangent) {
         const bool trajectory = taped && s->tape_traj;

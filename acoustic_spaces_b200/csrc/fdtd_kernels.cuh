@@ -541,7 +541,7 @@ struct Tables {
     // field its scale.
     uint32_t layer_quads, layer_lanes;
     const uint4 *layer_quad;
-    const uint32_t *lane_cell;
+    const uint32_t *lane_cell, *cell_lane;
     const float *lane_scale;
     uint32_t plane;  // pitch * ny
     FastDiv by_plane, by_pitch;  // a pitched index's plane, and its row within the plane
@@ -578,7 +578,7 @@ struct Fields {
     T *traj_u;         // when not null: each special row's new pressure at traj_u[k] (the gradient's
     T *traj_w;         // recomputation), and each branch state's new velocity at traj_w[j]
     // When not null (the gradient's recomputation of a grid with a matched layer): each layer
-    // cell's six factors per axis of the tables' gradient, at traj_layer[f * layers + c]
+    // cell's six factors per axis of the tables' gradient, at traj_layer[f * layer_lanes + its lane]
     // (fdtd_adjoint.cuh: q, hi' - lo', hi, b_(i+st) - b_i, lo, b_i - b_(i-st) per axis).
     T *traj_layer;
     // When not null (a run recording for a gradient along a tangent of the layer's tables): each
@@ -855,14 +855,30 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
     const T left = b[i - 1], right = b[i + 4];
     const uint32_t z = g.by_plane(i), r = i - z * g.plane, y = g.by_pitch(r), x = r - y * g.pitch;
     const Quad<T> sc = scales<T, SCALED>(g.lane_scale, 4 * q);
-    const bool recording = f.traj_layer || f.traj_tangent;
-    Quad<T> total{};
+    const bool recording = f.traj_tangent;
+    Quad<T> total{}, rise;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const uint32_t at = a == 0 ? x : (a == 1 ? y : z);
         float4 c[5];
 #pragma unroll
         for (int j = 0; j < (a == 0 ? 5 : 2); ++j) c[j] = a == 0 ? coef[0][(j % 4) * g.x_quads + x / 4 + j / 4] : coef[a][at + j];
+        // The step's factors of the tables' gradient, a quad each (a cell at a time they took 13.5 of the
+        // 22 us of a recorded step of 0.32M layer cells).
+        T *factors = f.traj_layer ? f.traj_layer + (uint64_t)(6 * a) * g.layer_lanes + 4 * (uint64_t)q : nullptr;
+        if (factors) {
+            Quad<T> up, down;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                up.v[j] = (a == 0 ? (j == 3 ? right : h.v[j + 1]) : (a == 1 ? yp.v[j] : zp.v[j])) - h.v[j];
+                down.v[j] = h.v[j] - (a == 0 ? (j == 0 ? left : h.v[j - 1]) : (a == 1 ? ym.v[j] : zm.v[j]));
+            }
+            store_quad<true>(factors, s.part[a]);
+            store_quad<true>(factors + 2 * (uint64_t)g.layer_lanes, s.hi[a]);
+            store_quad<true>(factors + 3 * (uint64_t)g.layer_lanes, up);
+            store_quad<true>(factors + 4 * (uint64_t)g.layer_lanes, s.lo[a]);
+            store_quad<true>(factors + 5 * (uint64_t)g.layer_lanes, down);
+        }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const float4 c0 = a == 0 ? c[j] : c[0], c1 = a == 0 ? c[j + 1] : c[1];
@@ -874,7 +890,7 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
             const T above = (T)c1.z * old_above - (T)c1.w * (hi - here);
             if (recording && (mask & (1u << j))) {
                 const uint32_t cell = g.lane_cell[4 * (uint64_t)q + j];
-                const uint32_t axes = f.traj_tangent ? g.tangent_axes[cell] : 0u;
+                const uint32_t axes = g.tangent_axes[cell];
                 if (axes & (1u << a)) {
                     // The step's factors along the tangent: its products with the adjoints of the new
                     // part and faces give the gradient's step (fdtd_adjoint.cuh), in double.
@@ -886,17 +902,8 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
                     o[1] = (T)((double)old_above * t1.x - (double)(hi - here) * t1.y);
                     o[2] = (T)((double)old_below * t0.x - (double)(here - lo) * t0.y);
                 }
-                if (f.traj_layer) {
-                    const uint64_t L = g.layers;
-                    T *o = f.traj_layer + (uint64_t)(6 * a) * L + cell;
-                    o[0] = before;
-                    o[1 * L] = above - below;
-                    o[2 * L] = old_above;
-                    o[3 * L] = hi - here;
-                    o[4 * L] = old_below;
-                    o[5 * L] = here - lo;
-                }
             }
+            rise.v[j] = above - below;
             const T push = SCALED ? (T)c0.y * sc.v[j] : (T)c0.y;
             const T flux = push * (above - below);
             if (COMP) {
@@ -909,6 +916,7 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
             }
             s.lo[a].v[j] = below, s.hi[a].v[j] = above;
         }
+        if (factors) store_quad<true>(factors + g.layer_lanes, rise);
     }
     if (COMP) {
         Quad<T> next;
@@ -935,7 +943,7 @@ __device__ __forceinline__ void layer_quad(const Tables &g, const Fields<T> &f, 
 // quads q, q + the grid's threads, ...; the next quad's entry is loaded while this one's loads are
 // in flight, so that a quad costs one round trip to memory rather than two.
 template <typename T, bool SCALED, bool COMP = false>
-__global__ void __launch_bounds__(kBlock) layer_kernel(const Tables g, const Fields<T> f) {
+__global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? 4 : 3) layer_kernel(const Tables g, const Fields<T> f) {
     const uint32_t n = g.layer_quads;
     const uint32_t step = gridDim.x * kBlock;
     uint32_t q = blockIdx.x * kBlock + threadIdx.x;

@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kResidentThreads<T, WIDE, LAYER>, 1)
         f.wb = cur ? p.w[1] : p.w[0], f.wa = cur ? p.w[0] : p.w[1], f.d = p.d;
         f.signal = p.signal + k;
         if (p.traj_u) f.traj_u = p.traj_u + (uint64_t)k * g.specials, f.traj_w = p.traj_w + (uint64_t)k * p.states;
-        if (LAYER && p.traj_layer) f.traj_layer = p.traj_layer + (uint64_t)k * 18 * g.layers;
+        if (LAYER && p.traj_layer) f.traj_layer = p.traj_layer + (uint64_t)k * 18 * g.layer_lanes;
         if (LAYER && p.traj_tangent) f.traj_tangent = p.traj_tangent + (uint64_t)k * p.tangent_factors;
         uint4 here = first;
         for (uint32_t t = warp; t < all; t += kWarps) {
