@@ -16,6 +16,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <future>
 #include <new>
 #include <string>
 
@@ -26,6 +27,7 @@
 #include "fdtd_adjoint.cuh"
 #include "fdtd_b200.h"
 #include "fdtd_flow.cuh"
+#include "fdtd_cluster.cuh"
 #include "fdtd_columns.cuh"
 #include "fdtd_kernels.cuh"
 #include "fdtd_resident.cuh"
@@ -58,6 +60,7 @@ constexpr uint64_t kGraphSteps = 64;  // steps of fdtd_run's captured chunk (eve
 // the graph: a step's launches and event waits cost as much host time as it takes on the device.
 constexpr uint64_t kGraphCells = 1ull << 23;
 constexpr uint32_t kResidentSmem = 216 * 1024;  // shared memory a block of the resident stepper takes at most
+constexpr uint64_t kClusterCells = 1ull << 16;  // (pitched) cells that a cluster's shared memory may take, to try
 constexpr uint64_t kGatheredSteps = 1024;  // steps the probes' cells are gathered over at most (even)
 
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -169,6 +172,13 @@ struct fdtd_solver {
     uint32_t resident_keep_layer = 0, resident_rows_at = 0, resident_layer_at = 0;
     const uint32_t *link_start = nullptr;
     const uint2 *row_links = nullptr;
+    // The smallest grids' cluster (fdtd_cluster.cuh): the rows and quads by owner and where the parts of a
+    // block's shared memory begin.
+    bool cluster_ready = false;
+    const uint4 *cluster_rows = nullptr;
+    const uint2 *cluster_quads = nullptr;
+    uint32_t cluster_row_start[17] = {}, cluster_quad_start[17] = {}, cluster_cells = 0, cluster_smem = 0;
+    uint32_t cluster_at[5] = {}, cluster_most[3] = {}, cluster_probe_steps = 1;  // links, states, rows, drive, reads; rows, states, reads
     // The launched sweep's columns (null: bulk_kernel's tiles, as fdtd_set_tiles has chosen).
     const uint2 *sweep_columns = nullptr;
     uint32_t sweep_count = 0;
@@ -531,8 +541,8 @@ void interior_columns(const fdtd_solver *s, const std::vector<uint8_t> &types, u
                     uint32_t four;
                     std::memcpy(&four, row + 4 * q, 4);
                     if (!four) continue;
-                    uint32_t mask = 0;
-                    for (int j = 0; j < 4; ++j) mask |= (((four >> (8 * j)) & 255u) == kInterior ? 1u : 0u) << j;
+                    uint32_t mask = four == 0x01010101u * kInterior ? 15u : 0u;
+                    if (!mask) for (int j = 0; j < 4; ++j) mask |= (((four >> (8 * j)) & 255u) == kInterior ? 1u : 0u) << j;
                     masks[q] |= mask << (4 * (z - z0));
                 }
             }
@@ -542,6 +552,13 @@ void interior_columns(const fdtd_solver *s, const std::vector<uint8_t> &types, u
                 columns.push_back(make_uint2((uint32_t)(plane * (z0 + skip) + s->pitch * y + 4 * q), masks[q] >> (4 * skip)));
             }
         }
+}
+
+template <typename V>
+int download(fdtd_solver *s, const V *device, size_t count, std::vector<V> &host) {
+    host.resize(count);
+    if (count) CUDA_TRY(s, cudaMemcpy(host.data(), device, count * sizeof(V), cudaMemcpyDeviceToHost));
+    return FDTD_OK;
 }
 
 // Planes a column of the launched sweep spans at most: a longer one reads the planes beyond its ends for
@@ -1035,7 +1052,30 @@ int launch_resident(fdtd_solver *s, const float *d_signal, uint64_t steps, doubl
         a.steps = (uint32_t)count;
         a.clustered = s->resident_clustered ? 1 : 0;
         a.arrived = s->arrived, a.error = s->d_error;
-        const int launched = launch_together(s, resident_kernel<T, WIDE, SCALED, COMP, LAYER>, s->resident_blocks,
+        int launched = FDTD_OK;
+        bool clustered = false;
+        if constexpr (!WIDE && !LAYER) {
+            if ((clustered = s->cluster_ready)) {
+                ClusterArgs<T> c{};
+                c.g = s->tables, c.air = a.air;
+                c.air.columns = s->cluster_quads;
+                for (int k = 0; k < 2; ++k) c.u[k] = a.u[k], c.w[k] = a.w[k];
+                c.cells = (uint32_t)s->n_device, c.own_cells = s->cluster_cells;
+                c.rows = s->cluster_rows;
+                for (int k = 0; k < 17; ++k) c.row_start[k] = s->cluster_row_start[k], c.quad_start[k] = s->cluster_quad_start[k];
+                c.link_start = s->link_start, c.links = s->row_links;
+                c.links_at = s->cluster_at[0], c.states_at = s->cluster_at[1], c.rows_at = s->cluster_at[2];
+                c.drive_at = s->cluster_at[3], c.reads_at = s->cluster_at[4];
+                c.most_rows = s->cluster_most[0], c.most_states = s->cluster_most[1], c.most_reads = s->cluster_most[2];
+                c.probe_steps = s->cluster_probe_steps;
+                c.signal = a.signal, c.gathered = a.gathered, c.gathered_count = a.gathered_count;
+                c.traj_u = a.traj_u, c.traj_w = a.traj_w, c.states = a.states, c.steps = a.steps;
+                launched = launch_together(s, cluster_kernel<T, SCALED, COMP>, kClusterBlocks, kClusterThreads<T>, s->cluster_smem,
+                                           true, c);
+            }
+        }
+        if (!clustered)
+            launched = launch_together(s, resident_kernel<T, WIDE, SCALED, COMP, LAYER>, s->resident_blocks,
                                              kResidentThreads<T, WIDE, LAYER>, s->resident_smem, s->resident_clustered, a);
         if (launched != FDTD_OK) return launched;
         if (probes && s->gathered_count) {
@@ -1092,10 +1132,78 @@ bool takes_resident(const fdtd_solver *s, const fdtd_layout *L) {
 }
 
 // The resident stepper's launch and lists for the grid, once takes_resident has said yes.
+// The smallest grids' cluster: 16 blocks, runs of cells going round them, the rows and quads (a plane each) by
+// their owner.
+template <typename T, bool SCALED, bool COMP>
+int set_up_cluster(fdtd_solver *s, const std::vector<uint32_t> &link_start, const std::vector<uint32_t> &state_start) {
+    if (s->n_device > kClusterCells) return FDTD_OK;
+    constexpr uint64_t a_round = (uint64_t)kClusterBlocks << kClusterRun;
+    const uint64_t own_cells = (s->n_device + a_round - 1) / a_round << kClusterRun;
+    const uint32_t K = (uint32_t)s->specials;
+    std::vector<uint32_t> special;
+    int rc;
+    if ((rc = download(s, s->tables.special, K, special))) return rc;
+    std::vector<std::vector<uint4>> rows(kClusterBlocks);
+    uint32_t links[kClusterBlocks] = {}, states[kClusterBlocks] = {};
+    for (uint32_t k = 0; k < K; ++k) {
+        const uint32_t owner = cluster_owner(special[k]), n = link_start[k + 1] - link_start[k], m = state_start[k + 1] - state_start[k];
+        if (m > 255) return FDTD_OK;
+        rows[owner].push_back(make_uint4(k, links[owner], states[owner], n | m << 8));
+        links[owner] += n, states[owner] += m;
+    }
+    std::vector<uint2> every, quads;
+    interior_columns(s, s->host_types, 1, every);
+    uint32_t most_rows = 0, most_links = 0, most_states = 0, most_tasks = 0;
+    std::vector<uint4> list;
+    for (uint32_t b = 0; b < kClusterBlocks; ++b) {
+        s->cluster_row_start[b] = (uint32_t)list.size(), s->cluster_quad_start[b] = (uint32_t)quads.size();
+        list.insert(list.end(), rows[b].begin(), rows[b].end());
+        for (const uint2 &q : every)
+            if (cluster_owner(q.x) == b) quads.push_back(q);
+        s->cluster_row_start[b + 1] = (uint32_t)list.size(), s->cluster_quad_start[b + 1] = (uint32_t)quads.size();
+        most_rows = std::max<uint32_t>(most_rows, (uint32_t)rows[b].size());
+        most_tasks = std::max<uint32_t>(most_tasks, ((uint32_t)rows[b].size() + 31) / 32 * 32 + s->cluster_quad_start[b + 1] - s->cluster_quad_start[b]);
+        most_links = std::max(most_links, links[b]), most_states = std::max(most_states, states[b]);
+    }
+    // A block's rows and quads, one a thread, up to three quarters of its threads in single precision, half in
+    // double. (Boxes of 12, 18, 22 and 28 cells a side, two branch states a row, us a step resident and in the
+    // cluster: 1.87 and 1.24, 2.02 and 1.58, 2.22 and 1.82, 2.62 and 2.20; 30 a side and four branches 3.60 and 4.57, 34 and no
+    // branches 2.29 and 3.50. In double 12, 14, 18 and 22: 1.74 and 1.53, 1.77 and 1.60, 2.03 and 2.04, 2.51 and 2.76: the
+    // other blocks' shared memory serves half as many of them.)
+    if (most_tasks > (sizeof(T) == 8 ? kClusterThreads<T> / 2 : kClusterThreads<T> / 4 * 3)) return FDTD_OK;
+    const uint64_t reads = (s->gathered_count + kClusterBlocks - 1) / kClusterBlocks;
+    s->cluster_probe_steps = (uint32_t)std::min<uint64_t>(64, reads ? (32u << 10) / (reads * sizeof(T)) : 64);
+    if (s->cluster_probe_steps < 4) return FDTD_OK;  // (a plane of receivers: the writes would hold the steps up)
+    auto up = [](uint64_t v) { return (v + 127) / 128 * 128; };
+    uint64_t at = up((uint64_t)kClusterCellBytes<T, SCALED, COMP> * own_cells);
+    const uint64_t parts[5] = {8ull * most_links, (16ull + 2 * sizeof(T)) * most_states, 36ull * most_rows, 4ull * kGatheredSteps,
+                               reads * sizeof(T) * s->cluster_probe_steps};
+    for (int k = 0; k < 5; ++k) s->cluster_at[k] = (uint32_t)at, at = up(at + parts[k]);
+    if (at > kResidentSmem) return FDTD_OK;
+    s->cluster_smem = (uint32_t)at, s->cluster_cells = (uint32_t)own_cells;
+    s->cluster_most[0] = most_rows, s->cluster_most[1] = most_states, s->cluster_most[2] = (uint32_t)reads;
+    auto kernel = cluster_kernel<T, SCALED, COMP>;
+    CUDA_TRY(s, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResidentSmem));
+    CUDA_TRY(s, cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t config = together(s, kClusterBlocks, kClusterThreads<T>, s->cluster_smem, true, attr);
+    int clusters = 0;
+    CUDA_TRY(s, cudaOccupancyMaxActiveClusters(&clusters, kernel, &config));
+    if (clusters < 1) return FDTD_OK;
+    if ((rc = upload(s, list.data(), list.size(), &s->cluster_rows))) return rc;
+    if ((rc = upload(s, quads.data(), quads.size(), &s->cluster_quads))) return rc;
+    s->cluster_ready = true;
+    return FDTD_OK;
+}
+
 template <typename T, bool WIDE, bool SCALED, bool COMP, bool LAYER>
 int set_up_resident(fdtd_solver *s, const std::vector<uint32_t> &link_start, const std::vector<uint32_t> &state_start) {
     s->resident = false;
     if (LAYER && 16 * (s->pitch + s->ny + s->nz + 6) > kResidentSmem) return FDTD_OK;  // (a grid of lines)
+    if constexpr (!WIDE && !LAYER) {
+        const int rc = set_up_cluster<T, SCALED, COMP>(s, link_start, state_start);
+        if (rc != FDTD_OK) return rc;
+    }
     auto kernel = resident_kernel<T, WIDE, SCALED, COMP, LAYER>;
     const int threads = kResidentThreads<T, WIDE, LAYER>;
     auto tasks = [](uint64_t n) { return (n + 31) / 32; };
@@ -1280,6 +1388,39 @@ int set_up_flow(fdtd_solver *s, const fdtd_layout *L) {
     return FDTD_OK;
 }
 
+// The matched layer's quads: those that hold layer cells, or the cells below them, in the grid's order, each
+// with the quads below it and its masks; each cell's lane (layer_lane), and each lane's cell (returned).
+std::vector<uint32_t> layer_lists(fdtd_solver *s, const fdtd_layout *L) {
+    const uint64_t Lc = L->layer_count, nx = L->nx, ny = L->ny;
+    std::vector<uint32_t> &cells = s->layer_cells;
+    cells.resize(Lc);
+    for (uint64_t c = 0; c < Lc; ++c) cells[c] = pitched(s, (uint64_t)L->layer_cells[c]);
+    std::vector<uint32_t> quad_of(s->n_device / 4, UINT32_MAX);
+    const uint32_t strides[3] = {1, (uint32_t)s->pitch, (uint32_t)(s->pitch * ny)};
+    for (const uint32_t i : cells) {
+        quad_of[i / 4] = 0;
+        for (const uint32_t stride : strides) quad_of[(i - stride) / 4] = 0;
+    }
+    std::vector<uint4> &quads = s->layer_quads;
+    for (uint64_t q = 0; q < quad_of.size(); ++q)
+        if (!quad_of[q]) quad_of[q] = (uint32_t)quads.size(), quads.push_back(make_uint4((uint32_t)(4 * q), 0, 0, 0));
+    if (quads.size() >= (1ull << 30)) return {};  // (refused)
+    std::vector<uint32_t> lane_cell(4 * quads.size(), 0);
+    s->layer_lane.resize(Lc);
+    for (uint64_t c = 0; c < Lc; ++c) {
+        const uint32_t i = cells[c], q = quad_of[i / 4], j = i % 4;
+        uint4 &entry = quads[q];
+        entry.y = quad_of[(i - strides[1]) / 4], entry.z = quad_of[(i - strides[2]) / 4];
+        entry.w |= 1u << j;
+        const uint64_t l = (uint64_t)L->layer_cells[c], below[3] = {1, nx, nx * ny};
+        for (int axis = 0; axis < 3; ++axis)
+            if (L->types[l - below[axis]] == kLayer) entry.w |= 1u << (4 + 4 * axis + j);
+        s->layer_lane[c] = 4 * q + j;
+        lane_cell[4 * (uint64_t)q + j] = (uint32_t)c;
+    }
+    return lane_cell;
+}
+
 int build(fdtd_solver *s, const fdtd_layout *L) {
     const uint64_t nx = L->nx, ny = L->ny, nz = L->nz, n = nx * ny * nz;
     s->nx = nx, s->ny = ny, s->nz = nz, s->n = n;
@@ -1301,6 +1442,10 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
     for (int k = 0; k < 18; ++k)
         g.offset[k] = (int32_t)(kSteps[k][0] + kSteps[k][1] * (int64_t)s->pitch + kSteps[k][2] * (int64_t)(s->pitch * ny));
 
+    // (The matched layer's lists beside the rest of the set-up; on this thread where there is no other.)
+    std::future<std::vector<uint32_t>> lists;
+    if (L->layer_count) lists = std::async(layer_lists, s, L);
+
     // Cell types and scales, pitched; the interior cells' bounding box and the air count.
     std::vector<uint8_t> types(s->n_device, (uint8_t)kSolid);
     std::vector<float> scale(s->scaled ? s->n_device : 0, 0.0f);
@@ -1310,15 +1455,17 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
             const uint64_t row = nx * (y + ny * z), drow = s->pitch * (y + ny * z);
             std::memcpy(&types[drow], &L->types[row], nx);
             if (s->scaled) std::memcpy(&scale[drow], &L->scale[row], nx * sizeof(float));
-            for (uint64_t x = 0; x < nx; ++x) {
-                const uint8_t t = L->types[row + x];
-                if (t != kSolid) ++air;
-                if (t != kInterior) continue;
-                ++interior;
-                x0 = std::min(x0, x), x1 = std::max(x1, x + 1);
-                y0 = std::min(y0, y), y1 = std::max(y1, y + 1);
-                z0 = std::min(z0, z), z1 = std::max(z1, z + 1);
-            }
+            const uint8_t *t = &L->types[row];
+            uint32_t open = 0, inner = 0;  // (sums that the compiler takes by vectors)
+            for (uint64_t x = 0; x < nx; ++x) open += t[x] != kSolid, inner += t[x] == kInterior;
+            air += open, interior += inner;
+            if (!inner) continue;
+            uint64_t first = 0, last = nx;
+            while (t[first] != kInterior) ++first;
+            while (t[last - 1] != kInterior) --last;
+            x0 = std::min(x0, first), x1 = std::max(x1, last);
+            y0 = std::min(y0, y), y1 = std::max(y1, y + 1);
+            z0 = std::min(z0, z), z1 = std::max(z1, z + 1);
         }
     s->interior = interior, s->air = air;
 
@@ -1448,7 +1595,7 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
             if ((rc = upload(s, mask.data(), K, &u8))) return rc;
             g.link_mask = u8;
         }
-        if (!axial_rows && resident) {
+        if (resident) {
             // The resident stepper's links, row by row.
             std::vector<uint2> links(L->link_count);
             for (uint64_t l = 0; l < L->link_count; ++l) {
@@ -1500,36 +1647,13 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
     s->layers = Lc;
     g.layers = (uint32_t)Lc;
     if (Lc) {
-        std::vector<uint32_t> cells(Lc);
-        for (uint64_t c = 0; c < Lc; ++c) cells[c] = pitched(s, (uint64_t)L->layer_cells[c]);
-        s->layer_cells = cells;
+        const std::vector<uint32_t> lane_cell = lists.get();
+        const std::vector<uint32_t> &cells = s->layer_cells;
+        const std::vector<uint4> &quads = s->layer_quads;
         const uint32_t *p;
         if ((rc = upload(s, cells.data(), Lc, &p))) return rc;
         g.layer_cells = p;
-        // The quads that hold layer cells, or the cells below them, in the grid's order.
-        std::vector<uint32_t> quad_of(s->n_device / 4, UINT32_MAX);
-        const uint32_t strides[3] = {1, g.pitch, g.plane};
-        for (const uint32_t i : cells) {
-            quad_of[i / 4] = 0;
-            for (const uint32_t stride : strides) quad_of[(i - stride) / 4] = 0;
-        }
-        std::vector<uint4> &quads = s->layer_quads;
-        for (uint64_t q = 0; q < quad_of.size(); ++q)
-            if (!quad_of[q]) quad_of[q] = (uint32_t)quads.size(), quads.push_back(make_uint4((uint32_t)(4 * q), 0, 0, 0));
         if (quads.size() >= (1ull << 30)) return fail(s, FDTD_EINVAL, "the matched layer is too large for the GPU's 32-bit indices");
-        std::vector<uint32_t> lane_cell(4 * quads.size(), 0);
-        s->layer_lane.resize(Lc);
-        for (uint64_t c = 0; c < Lc; ++c) {
-            const uint32_t i = cells[c], q = quad_of[i / 4], j = i % 4;
-            uint4 &entry = quads[q];
-            entry.y = quad_of[(i - strides[1]) / 4], entry.z = quad_of[(i - strides[2]) / 4];
-            entry.w |= 1u << j;
-            const uint64_t l = (uint64_t)L->layer_cells[c], below[3] = {1, nx, nx * ny};
-            for (int axis = 0; axis < 3; ++axis)
-                if (L->types[l - below[axis]] == kLayer) entry.w |= 1u << (4 + 4 * axis + j);
-            s->layer_lane[c] = 4 * q + j;
-            lane_cell[4 * (uint64_t)q + j] = (uint32_t)c;
-        }
         g.layer_quads = (uint32_t)quads.size(), g.layer_lanes = 4 * g.layer_quads;
         if ((rc = upload(s, quads.data(), quads.size(), &g.layer_quad))) return rc;
         if ((rc = upload(s, lane_cell.data(), lane_cell.size(), &g.lane_cell))) return rc;
@@ -1619,13 +1743,6 @@ void release(fdtd_solver *s) {
 // ---------------------------------------------------------------------------------------------
 // The adjoint (see fdtd_adjoint.cuh)
 // ---------------------------------------------------------------------------------------------
-
-template <typename V>
-int download(fdtd_solver *s, const V *device, size_t count, std::vector<V> &host) {
-    host.resize(count);
-    if (count) CUDA_TRY(s, cudaMemcpy(host.data(), device, count * sizeof(V), cudaMemcpyDeviceToHost));
-    return FDTD_OK;
-}
 
 // The adjoint's tables on the host: the readers of each special row's cell (the transposed links)
 // and the interior cells next to special rows with their corrections.
@@ -2583,7 +2700,10 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
 // only through the address cudaGetSymbolAddress gives (pool_address).
 constexpr size_t kPoolBytes = FDTD_GRADIENT_STATIC_BYTES;
 constexpr size_t kPoolAlign = 256;
-static __device__ __align__(256) unsigned char g_gradient_pool[kPoolBytes];
+// A gradient is taken when its buffers by cells fit kPoolBytes. The layer's factors lie by its quads' lanes, of
+// which there are 1.1 to 1.3 a cell in layers of eight cells and up to 4 in layers of one: the pool has room for them.
+constexpr size_t kPoolRoom = 4 * kPoolBytes;
+static __device__ __align__(256) unsigned char g_gradient_pool[kPoolRoom];
 
 constexpr size_t pool_round(size_t bytes) { return ((bytes ? bytes : 16) + kPoolAlign - 1) / kPoolAlign * kPoolAlign; }
 
@@ -2609,7 +2729,7 @@ struct StaticPool {
     int take(size_t bytes, void **out, bool zero) {
         *out = nullptr;
         const size_t size = pool_round(bytes);
-        if (used + size > kPoolBytes) return fail(s, FDTD_EINVAL, "the gradient's buffers outgrow the static pool");
+        if (used + size > kPoolRoom) return fail(s, FDTD_EINVAL, "the gradient's buffers outgrow the static pool");
         *out = base + used;
         used += size;
         if (zero) CUDA_TRY(s, cudaMemsetAsync(*out, 0, size, s->stream));
@@ -2619,8 +2739,10 @@ struct StaticPool {
 };
 
 // The pool's bytes for one gradient: the blocks place_adjoint and then gradient<T> take, in order
-// (the checkpoints only where no tape supplies the segments' states).
-size_t pool_bytes(const fdtd_solver *s, const AdjointLists &l, uint64_t steps, uint64_t segment, bool taped) {
+// (the checkpoints only where no tape supplies the segments' states), the layer's factors `lanes` a step and axis,
+// its state `slots` a checkpoint.
+size_t pool_bytes(const fdtd_solver *s, const AdjointLists &l, uint64_t steps, uint64_t segment, bool taped, uint64_t lanes,
+                  uint64_t slots) {
     const size_t e = s->precision == FDTD_FP64 ? 8 : 4;
     const uint64_t K = s->specials, S = s->states, P = std::max<uint64_t>(1, s->probes), n = s->n_device;
     size_t total = 0;
@@ -2645,7 +2767,7 @@ size_t pool_bytes(const fdtd_solver *s, const AdjointLists &l, uint64_t steps, u
     total += 2 * pool_round(8 * K) + 3 * pool_round(8 * S);
     if (Lc) total += pool_round(4 * l.by_coord.size()) + pool_round(4 * l.coord_start.size());
     if (Lc && s->gradient_tables && !s->tangent)
-        total += pool_round(e * kLayerFactors * s->tables.layer_lanes * segment) + pool_round(8 * kLayerFactors * Lc) +
+        total += pool_round(e * kLayerFactors * lanes * segment) + pool_round(8 * kLayerFactors * Lc) +
                  pool_round(8 * 6 * (s->nx + s->ny + s->nz));
     if (Lc && s->tangent) {
         const bool trajectory = taped && s->tape_traj;
@@ -2653,7 +2775,7 @@ size_t pool_bytes(const fdtd_solver *s, const AdjointLists &l, uint64_t steps, u
         if (!trajectory) total += pool_round(e * s->tangent_factors * segment);
         total += pool_round(8 * Lc) + pool_round(8 * (blocks + 1)) + pool_round(sizeof(void *));
     }
-    if (!taped) total += (segments - 1) * pool_round(checkpoint_bytes(s));
+    if (!taped) total += (segments - 1) * pool_round(2 * e * (n + S) + e * kLayerSlots * slots);
     return total;
 }
 
@@ -2975,8 +3097,10 @@ int fdtd_gradient_noalloc(fdtd_solver *s, const float *signal, uint64_t steps, c
     if ((rc = pool_address(s, &base)) != FDTD_OK) return rc;
     AdjointLists lists;
     if ((rc = adjoint_lists(s, lists)) != FDTD_OK) return rc;
-    const size_t need = pool_bytes(s, lists, steps, segment, holds_tape(s, signal, steps, segment));
-    if (need > kPoolBytes) {
+    const bool taped = holds_tape(s, signal, steps, segment);
+    const uint64_t lanes = s->tables.layer_lanes;
+    const size_t need = pool_bytes(s, lists, steps, segment, taped, s->layers, s->layers ? s->n_device : 0);
+    if (need > kPoolBytes || pool_bytes(s, lists, steps, segment, taped, lanes, lanes) > kPoolRoom) {
         char message[200];
         std::snprintf(message, sizeof message,
                       "the gradient needs %llu bytes of device memory; the static pool holds %llu: fewer steps, a "

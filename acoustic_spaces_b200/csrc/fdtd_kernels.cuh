@@ -1,5 +1,7 @@
 // Device code of the B200 wave stepper: one time step of WaveSolver::run
-// (cpp/include/acoustic_spaces/fdtd.hpp:786-904 of naelolaiz/acoustic-spaces) as four kernels.
+// (cpp/include/acoustic_spaces/fdtd.hpp:786-904 of naelolaiz/acoustic-spaces) by a kernel a kind of
+// work. (fdtd_columns.cuh: the interior sweep that is launched; fdtd_resident.cuh: all kinds and many
+// steps in one launch, for the smaller grids.)
 //
 // A step reads the current pressure b and branch velocities wb, and writes the next pressure over
 // the previous one in a, the branch velocities over wa and the matched layer's state in place.
@@ -592,8 +594,8 @@ struct Fields {
 // are coalesced; all of a row's loads — its links' pressures and weights, its coefficients and its
 // first branch state — are issued before the sum, which then adds the links in the layout's order: a
 // row waits once for memory (its cell and its links' directions come with the row before), where
-// directions before pressures before states took three waits (the fitted rows of the 4 cm room:
-// 64.0 us with them, 74.1 at 8 blocks an SM before; see special_kernel). A state's term now * wb -
+// directions before pressures before states took three waits (the fitted rows of the 4 cm room,
+// timed alone: 74.1 us so, 53.8 with one). A state's term now * wb -
 // before * wa is worked out again for the velocities' update rather than kept: wa has not changed in
 // between, so it is the same value.
 // The links' tables are read once a step and the new pressure by no kernel of the same step, so

@@ -302,9 +302,9 @@ class B200WaveSolver:
 
     def autotune(self, trial_steps: int = 12) -> dict[str, int]:
         """Chooses the launch shapes for this grid by timing a few steps of each candidate (from
-        rest; the state is reset after): the interior sweep's tile shape and planes a tile, then
-        the matched-layer and special-row kernels' blocks per multiprocessor. Returns the choice
-        (blocks 0: one thread a cell; the tiles as :meth:`tiles` gives them)."""
+        rest; the state is reset after): the matched-layer and special-row kernels' blocks per
+        multiprocessor and the streams (and the sweep's tiles, where :meth:`set_tiles` has chosen
+        tiles). Returns the choice (blocks 0: one thread a row or quad of cells; the tiles as :meth:`tiles` gives them)."""
         layer, special = ctypes.c_int(), ctypes.c_int()
         status = self._lib.fdtd_autotune(self._handle, int(trial_steps), ctypes.byref(layer), ctypes.byref(special))
         if status != _abi.FDTD_OK:
@@ -312,8 +312,9 @@ class B200WaveSolver:
         return {"layer_blocks_per_sm": layer.value, "special_blocks_per_sm": special.value, **self.tiles()}
 
     def tiles(self) -> dict[str, int]:
-        """The interior sweep's tiles: shape index, cells a tile along x and y, ring stages,
-        planes a tile, tiles, resident blocks a multiprocessor and threads a block."""
+        """The interior sweep's tiles (used once :meth:`set_tiles` has chosen other ones): shape index,
+        cells a tile along x and y, ring stages, planes a tile, tiles, resident blocks a multiprocessor
+        and threads a block."""
         t = _abi.FdtdTiles()
         status = self._lib.fdtd_get_tiles(self._handle, ctypes.byref(t))
         if status != _abi.FDTD_OK:
@@ -341,7 +342,7 @@ class B200WaveSolver:
 
     def set_tiles(self, shape: int, planes: int) -> None:
         """Sets the interior sweep's tile shape (0: 64 x 16, 1: 128 x 16, 2: 64 x 32, 3: 32 x 32)
-        and planes a tile, as :meth:`autotune` would; results are the same to the bit."""
+        and planes a tile, in place of its columns; results are the same to the bit."""
         status = self._lib.fdtd_set_tiles(self._handle, int(shape), int(planes))
         if status != _abi.FDTD_OK:
             _raise(self._lib, status, self._handle)

@@ -261,19 +261,25 @@ int fdtd_set_tape_budget(fdtd_solver *solver, uint64_t bytes);
 
 /*
  * Chooses the launch shapes for this grid (no counterpart in the reference): from rest, steps
- * `trial_steps` steps (0: 8) with each candidate and keeps the fastest by CUDA events — first the
- * interior sweep's tile shape (each of the ten shapes of fdtd_tiles that fits a multiprocessor,
- * each with 1/4, 1/2, 1 and 2 times the default planes a tile, within 8 to 64), then, with the best
- * tiles, the count of blocks per multiprocessor of the matched-layer and special-row kernels and
- * the six arrangements of the step's kernels on the streams (fdtd_set_streams), then the tiles again; the
- * best few whole choices are timed three times more and the fastest kept — and resets the state.
+ * `trial_steps` steps (0: 8) with each candidate and keeps the fastest by CUDA events — the count
+ * of blocks per multiprocessor of the matched-layer and special-row kernels and the six
+ * arrangements of the step's kernels on the streams (fdtd_set_streams); where the interior is swept
+ * by tiles (after fdtd_set_tiles), first and then again the tiles' shape (each of the ten of
+ * fdtd_tiles that fits a multiprocessor, with 1/4, 1/2, 1 and 2 times the default planes a tile,
+ * within 8 to 64); the best few whole choices are timed three times more and the fastest kept — and
+ * resets the state. A grid whose steps run many to a launch keeps doing so: the choices are for its
+ * launched steps (fdtd_set_launch).
  * The chosen counts are written to *layer_per_sm and *special_per_sm when given (0: one thread a
  * cell); fdtd_get_tiles gives the rest. Results do not depend on any of these choices. Refused
  * after steps (fdtd_reset first).
  */
 int fdtd_autotune(fdtd_solver *solver, uint64_t trial_steps, int *layer_per_sm, int *special_per_sm);
 
-/* The interior sweep's tiles (no counterpart in the reference). */
+/*
+ * The interior sweep's tiles (no counterpart in the reference). The interior is swept by columns of
+ * quads of cells, which have no shape to choose; a handle takes these tiles once fdtd_set_tiles has
+ * chosen other ones than fdtd_get_tiles gives at first.
+ */
 typedef struct fdtd_tiles {
     int shape;          /* 0: 64 x 16 cells, 5 stages; 1: 128 x 16, 4; 2: 64 x 32, 4; 3: 32 x 32, 5 (128
                          * threads a block, a column a thread); 4, 5, 6: shapes 0, 1, 2 with 256
@@ -308,7 +314,8 @@ int fdtd_get_tiles(const fdtd_solver *solver, fdtd_tiles *out);
  * layer beside them; 0, all one after another on the handle's stream; 4 and 5, as 1 and 2 with
  * the special rows launched at the device's highest stream priority, so that their blocks run
  * beside the sweep's from the step's start. Results are the same to the bit. FDTD_EINVAL outside
- * 0 to 5. Waits for the handle's work.
+ * 0 to 5. Waits for the handle's work. (Small grids step many steps in one launch, which has no
+ * streams; this call, fdtd_set_launch and fdtd_set_tiles make a handle launch each step's kernels.)
  */
 int fdtd_set_streams(fdtd_solver *solver, int concurrent);
 
@@ -317,6 +324,7 @@ int fdtd_set_streams(fdtd_solver *solver, int concurrent);
  * and corrected cells far from the matched layer, `near_per_sm` for its launch of the rest and the
  * layer's cells (0: a block for every 128 of them; no counterpart in the reference). Fewer blocks
  * let the launches run beside one another and the interior sweep. Results are the same to the bit.
+ * (Small grids step back many steps in one launch; this call makes a handle launch each step's.)
  */
 int fdtd_set_adjoint_launch(fdtd_solver *solver, int far_per_sm, int near_per_sm);
 
@@ -375,7 +383,8 @@ int fdtd_set_launch(fdtd_solver *solver, int layer_per_sm, int special_per_sm);
 int fdtd_set_coefficients(fdtd_solver *solver, const float *coef_b, const float *coef_inv, const float *branch_now,
                           const float *branch_before, const float *branch_gain);
 
-/* Bytes of the static device pool of fdtd_gradient_noalloc: 16 MiB, held on every device the
+/* Bytes of the static device pool of fdtd_gradient_noalloc: 16 MiB, in 64 MiB (the matched layer's
+ * buffers are padded to whole quads of cells) held on every device the
    library runs on until the process exits. */
 #define FDTD_GRADIENT_STATIC_BYTES (16ull << 20)
 

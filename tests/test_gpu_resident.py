@@ -56,6 +56,14 @@ def test_gpu_boxes_of_odd_sizes_step_as_the_oracle_does(shape, speed, precision,
     _equal(_box(shape, speed=speed), _drive(steps), [0, 1, 34, steps], precision, launched)
 
 
+@pytest.mark.parametrize("precision", ["fp32", "fp64", "fp32c"])
+@pytest.mark.parametrize("shape, branches, speed", [((11, 12, 11), 0, None), ((18, 18, 18), 3, 0.95), ((28, 28, 28), 2, None), ((30, 29, 31), 4, None)])
+def test_gpu_grids_of_one_cluster_step_as_the_oracle_does(shape, branches, speed, precision):
+    """A block's tasks fewer than a warp's, planes a power of two apart, and both sides of the line to the whole GPU;
+    the probes written out within a run and at its end."""
+    _equal(_box(shape, speed=speed, branches=branches, receivers=1), _drive(203), [0, 1, 66, 203], precision)
+
+
 def test_gpu_runs_longer_than_a_launch():
     _equal(_box((12, 10, 13)), _drive(2111), [0, 1030, 1031, 2111], "fp32")
 
