@@ -1402,6 +1402,7 @@ std::vector<uint32_t> layer_lists(fdtd_solver *s, const fdtd_layout *L) {
         for (const uint32_t stride : strides) quad_of[(i - stride) / 4] = 0;
     }
     std::vector<uint4> &quads = s->layer_quads;
+    quads.reserve((size_t)std::count(quad_of.begin(), quad_of.end(), 0u));
     for (uint64_t q = 0; q < quad_of.size(); ++q)
         if (!quad_of[q]) quad_of[q] = (uint32_t)quads.size(), quads.push_back(make_uint4((uint32_t)(4 * q), 0, 0, 0));
     if (quads.size() >= (1ull << 30)) return {};  // (refused)
