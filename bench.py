@@ -1247,7 +1247,7 @@ def main() -> None:
             "gpu_launches": launches_per_step * steps + (-(-steps // 1024) if solver.probes else 0),
             "roofline": {
                 "bound": "hbm",
-                "kernel": f"{dominant}_kernel (the longest of the step's kernels, by CUDA events)",
+                "kernel": f"{'column' if dominant == 'bulk' else dominant}_kernel (the longest of the step's kernels, by CUDA events)",
                 "achieved": kernels[dominant]["achieved"],
                 "peak": peak,
                 "unit": "GB/s",
