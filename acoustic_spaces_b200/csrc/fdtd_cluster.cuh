@@ -2,11 +2,13 @@
 // a run in one launch.
 //
 // A step of a few thousand cells is all latency: through L2 it costs the pressures' round trip and the
-// barrier's, 2.4 us (the resident stepper's cluster). Here the pitched grid's runs of 64 cells go round the
-// blocks, so that the walls' rows are shared out evenly, and each block keeps both levels of them, its rows' tables and its branch velocities in shared memory;
-// a cell's neighbours are read from whichever block owns them (ld.shared::cluster), its new pressure is
-// written to its own block's, and the cluster's barrier ends the step. The operations of each cell are
-// the launched kernels', in their order.
+// barrier's (the resident stepper: 1.5-2.6 us). Here the pitched grid's runs of 64 cells go round the
+// blocks, so that the walls' rows are shared out evenly, and each block keeps both levels of its cells, its
+// rows' tables and its branch velocities in shared memory; a cell's neighbours are read from whichever block
+// owns them (ld.shared::cluster), its new pressure is written to its own block's, and the cluster's barrier
+// ends the step: 0.85 us on a plain box of 12 cells a side, 1.24 with two branch states a row, 2.2 at 28 a side
+// (a run of planes a block instead, the floor's rows on one block: 3.5). The operations of each cell are the
+// launched kernels', in their order.
 #pragma once
 
 #include "fdtd_resident.cuh"
@@ -68,7 +70,8 @@ struct ClusterArgs {
 
 // A block's shared memory: two levels (and the increments, and the scales), the links {weight, address of the
 // first level's cell in its owner}, the states {weight, now, before, gain} and their velocities, the rows {cell
-// within the block, row, first link | counts, first state}, their coefficients, the drive, and the probes' pressures of some steps.
+// within the block, row, first link | links << 24, first state | states << 24}, their coefficients, the drive, and
+// the probes' pressures of some steps.
 template <typename T, bool SCALED, bool COMP>
 constexpr uint32_t kClusterCellBytes = sizeof(T) * (COMP ? 3 : 2) + (SCALED ? 4 : 0);
 
