@@ -36,10 +36,6 @@ __device__ __forceinline__ void load_cluster(uint32_t at, Quad<double> &q) {
     asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(q.v[0]), "=d"(q.v[1]) : "r"(at) : "memory");
     asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(q.v[2]), "=d"(q.v[3]) : "r"(at + 16) : "memory");
 }
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-
 constexpr uint32_t kClusterBlocks = 16, kClusterRun = 6;
 // The block of cell i: runs of 64 cells go round the 16, each round five further on than the one before (walls a
 // power of two apart would else fall on a few blocks).

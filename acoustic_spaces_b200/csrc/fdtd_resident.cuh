@@ -43,13 +43,19 @@ struct ResidentArgs {
     unsigned int *error;
 };
 
+// Every thread of the cluster has arrived, and sees what the others wrote before they did. (Not the aligned form: it
+// wants a warp's threads together, and the loops before it end lane by lane.)
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
+}
+
 // Every block of the launch has done its part of a step: a count in device memory, cleared before
 // the launch (`target`: the blocks times the barriers so far), or the cluster's barrier. False
 // after too many tries: the block then reports the error and stops, and so do the others.
 __device__ __forceinline__ bool step_barrier(unsigned int *arrived, unsigned int target, uint32_t clustered,
                                              unsigned int *error) {
     if (clustered) {
-        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        cluster_barrier();
         return true;
     }
     int failed = 0;
