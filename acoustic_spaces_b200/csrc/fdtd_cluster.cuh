@@ -242,14 +242,20 @@ __global__ void __launch_bounds__(kClusterThreads<T>, 1) cluster_kernel(const __
             __syncthreads();
         }
     }
-    for (uint32_t c = threadIdx.x; c < own_cells; c += kThreads) {
-        const uint32_t i = global(c);
-        if (i >= p.cells) continue;
-        p.u[0][i] = level[c], p.u[1][i] = level[own_cells + c];
-        if (COMP) p.air.d[i] = increment[c];
+    // Back go the cells that the block steps and no others: a solid plane may be a neighbour's ghost plane, which a
+    // copy fills beside this launch.
+    for (uint32_t k = threadIdx.x; k < quads; k += kThreads) {
+        const uint2 q = p.air.columns[p.quad_start[rank] + k];
+        const uint32_t c = local(q.x);
+        store_cells<false>(p.u[0] + q.x, load_quad(level + c), q.y);
+        store_cells<false>(p.u[1] + q.x, load_quad(level + own_cells + c), q.y);
+        if (COMP) store_cells<false>(p.air.d + q.x, load_quad(increment + c), q.y);
     }
     for (uint32_t k = threadIdx.x; k < rows; k += kThreads) {
         const uint4 e = row[k];
+        const uint32_t i = g.special[e.y];
+        p.u[0][i] = level[e.x], p.u[1][i] = level[own_cells + e.x];
+        if (COMP) p.air.d[i] = increment[e.x];
         const uint32_t s0 = e.w & 0xffffffu, m = e.w >> 24, to = g.state_start[e.y];
         for (uint32_t j = 0; j < m; ++j) p.w[0][to + j] = w[s0 + j], p.w[1][to + j] = w[p.most_states + s0 + j];
     }
