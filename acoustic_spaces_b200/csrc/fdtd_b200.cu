@@ -802,8 +802,9 @@ int sum_probes(fdtd_solver *s, uint64_t steps, double *d_out, uint64_t stride) {
     return FDTD_OK;
 }
 
+// Steps done .. done + steps - 1 of a dispatch (the drive and the records the piece's own).
 template <typename T, bool WIDE, bool SCALED, bool COMP>
-int launch_piece(fdtd_solver *s, const float *d_signal, uint64_t steps, double *d_out, uint64_t stride) {
+int launch_piece(fdtd_solver *s, const float *d_signal, uint64_t done, uint64_t steps, double *d_out, uint64_t stride) {
     const Tables &g = s->tables;
     // The layer and special kernels loop over their cells: a few blocks an SM each (the handle's
     // layer_per_sm, special_per_sm; 0: a thread a cell), leaving the sweep's blocks their places.
@@ -857,15 +858,17 @@ int launch_piece(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
         f.out_stride = stride;
         f.gathered = static_cast<T *>(s->gathered) + k * gathered;
         f.gathered_count = gathered;
+        // The recordings are the whole dispatch's, whatever pieces it is launched in.
+        const uint64_t at = done + k;
         if (s->record_u) {
-            // The special rows' new values, level k + record_offset of the trajectory.
-            f.traj_u = static_cast<T *>(s->record_u) + (k + s->record_offset) * s->specials;
-            f.traj_w = static_cast<T *>(s->record_w) + (k + s->record_offset) * s->states;
+            // The special rows' new values, level at + record_offset of the trajectory.
+            f.traj_u = static_cast<T *>(s->record_u) + (at + s->record_offset) * s->specials;
+            f.traj_w = static_cast<T *>(s->record_w) + (at + s->record_offset) * s->states;
         }
-        // The matched layer's factors of step k (the gradient's recomputation).
-        if (s->record_layer) f.traj_layer = static_cast<T *>(s->record_layer) + k * kLayerFactors * g.layer_lanes;
-        // The factors of step k along the tables' tangent (a gradient's recomputation, or a taped run).
-        if (s->record_tangent) f.traj_tangent = static_cast<T *>(s->record_tangent) + k * s->tangent_factors;
+        // The matched layer's factors of the step (the gradient's recomputation).
+        if (s->record_layer) f.traj_layer = static_cast<T *>(s->record_layer) + at * kLayerFactors * g.layer_lanes;
+        // The factors of the step along the tables' tangent (a gradient's recomputation, or a taped run).
+        if (s->record_tangent) f.traj_tangent = static_cast<T *>(s->record_tangent) + at * s->tangent_factors;
         if (fork) {
             if (k > 0) {
                 CUDA_TRY(s, cudaStreamWaitEvent(s->stream, s->joined[1], 0));
@@ -949,13 +952,14 @@ int launch_piece(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
     return gathered ? sum_probes<T>(s, steps, d_out, stride) : FDTD_OK;
 }
 
-// The steps by a launch a kind of work, in pieces of at most gathered_steps steps (an even count: the
-// levels' roles return), each followed by its probes' sums.
+// The steps by a launch a kind of work; where probes' cells are gathered, in pieces of at most
+// gathered_steps steps (an even count: the levels' roles return), each followed by its probes' sums.
 template <typename T, bool WIDE, bool SCALED, bool COMP>
 int launch_steps(fdtd_solver *s, const float *d_signal, uint64_t steps, double *d_out, uint64_t stride) {
     for (uint64_t done = 0; done < steps;) {
-        const uint64_t count = std::min<uint64_t>(steps - done, s->gathered_steps);
-        const int rc = launch_piece<T, WIDE, SCALED, COMP>(s, d_signal + done, count, d_out + done, stride);
+        const bool gathers = s->probes && s->record_probes && !s->flowing;
+        const uint64_t count = gathers ? std::min<uint64_t>(steps - done, s->gathered_steps) : steps - done;
+        const int rc = launch_piece<T, WIDE, SCALED, COMP>(s, d_signal + done, done, count, d_out + done, stride);
         if (rc != FDTD_OK) return rc;
         done += count;
     }
