@@ -811,10 +811,11 @@ int launch_piece(fdtd_solver *s, const float *d_signal, uint64_t done, uint64_t 
     const uint64_t special_cap = s->special_per_sm ? (uint64_t)s->sms * s->special_per_sm : UINT64_MAX;
     const uint64_t layer_cap = s->layer_per_sm ? (uint64_t)s->sms * s->layer_per_sm : UINT64_MAX;
     const bool probes = s->probes && s->record_probes;
-    const uint32_t gathered = probes && !s->flowing ? s->gathered_count : 0;
+    // (A single step's probes are read beside its sweep: a call of one step took 2 us more with their sums after it.)
+    const uint32_t gathered = probes && !s->flowing && steps > 1 ? s->gathered_count : 0;
     const uint32_t special_blocks = (uint32_t)std::min<uint64_t>(
         (std::max<uint64_t>(s->specials, gathered) + kBlock - 1) / kBlock, special_cap);
-    const uint32_t probe_blocks = probes && s->flowing ? (uint32_t)((s->probes + kProbeWarps - 1) / kProbeWarps) : 0;
+    const uint32_t probe_blocks = probes && !gathered ? (uint32_t)((s->probes + kProbeWarps - 1) / kProbeWarps) : 0;
     const uint32_t layer_blocks = (uint32_t)std::min<uint64_t>((g.layer_quads + kBlock - 1) / kBlock, layer_cap);
     // Each step: the interior sweep on the handle's stream; beside it the matched layer on the
     // layer stream, of the highest priority (its blocks take the thread slots that the sweep's
@@ -937,6 +938,7 @@ int launch_piece(fdtd_solver *s, const float *d_signal, uint64_t done, uint64_t 
         }
         if (ev) CUDA_TRY(s, cudaEventRecord(ev[5], side));
         if (ev) CUDA_TRY(s, cudaEventRecord(ev[6], side));
+        if (probe_blocks && !s->flowing) probe_kernel<T><<<probe_blocks, kBlock, 0, side>>>(g, f);
         if (ev) CUDA_TRY(s, cudaEventRecord(ev[7], side));
         if (fork) {
             CUDA_TRY(s, cudaEventRecord(s->joined[1], side));
@@ -1093,7 +1095,10 @@ int launch_resident(fdtd_solver *s, const float *d_signal, uint64_t steps, doubl
 
 template <typename T, bool W, bool S, bool C>
 int dispatch_run(fdtd_solver *s, const float *d_signal, uint64_t steps, double *d_out, uint64_t stride) {
-    if (s->resident && !s->timing)
+    // (A single step is launched: the resident stepper's launch, which loads and stores each block's tables and state,
+    // took 14.4 to 20.9 us of one step on 2,000 to 870,000 cells, the launched kernels 12.4 to 16.6; two steps 16 to 27
+    // and 20 to 27.)
+    if (s->resident && !s->timing && steps > 1)
         return s->layers ? launch_resident<T, W, S, C, !W>(s, d_signal, steps, d_out, stride)
                          : launch_resident<T, W, S, C, false>(s, d_signal, steps, d_out, stride);
     return launch_steps<T, W, S, C>(s, d_signal, steps, d_out, stride);

@@ -5,13 +5,15 @@ from __future__ import annotations
 
 import numpy as np
 import pytest
+from conftest import load_golden
 
 from acoustic_spaces_b200 import B200WaveSolver, layouts
+from oracle.oracle import OracleSolver
 
 pytestmark = pytest.mark.gpu
 
 
-def _box(receivers=1):
+def _box():
     rng = np.random.default_rng(5)
     cell, rate = 0.1, 5000.0
     size = np.array([12, 9, 11]) * cell
@@ -30,9 +32,10 @@ def _repeated(layout, times):
                 probe_weights=np.tile(layout["probe_weights"], times))  # fmt: skip
 
 
-def _gradient(layout, precision, steps, segment, tape, *, tables=True, tangent=None):
+def _gradient(layout, precision, steps, segment, tape, *, tables=True, tangent=None, launched=True):
     solver = B200WaveSolver(layout, precision=precision)
-    solver.set_streams(1)  # each step's kernels launched
+    if launched:
+        solver.set_streams(1)  # each step's kernels launched
     if tangent is not None:
         solver.set_layer_tangent(tangent)
     if tape:
@@ -81,3 +84,29 @@ def test_gpu_layer_gradients_of_many_receivers(tape, kind):
     # (The tangent's products are added up a segment at a time in the step's own precision.)
     for key in a:
         np.testing.assert_allclose(a[key], b[key], rtol=1e-10, atol=1e-10 * np.abs(b[key]).max(), err_msg=key)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64", "fp32c"])
+@pytest.mark.parametrize("kind", ["box", "wide", "layer"])
+def test_gpu_single_steps_between_longer_runs(kind, precision):
+    if kind == "box":
+        layout = _box()
+    elif kind == "wide":
+        layout = load_golden("resonant19")[0]
+    else:
+        layout = layouts.polyhedral_room(2, cell=0.3, receivers=3, steps=1).built.layout
+    drive = np.random.default_rng(6).standard_normal(70).astype(np.float32)
+    solver, oracle = B200WaveSolver(layout, precision=precision), OracleSolver(layout, precision)
+    cuts = [0, 1, 2, 3, 20, 21, 23, 24, 25, 69, 70]
+    got = np.concatenate([solver.run(drive[i:j]) for i, j in zip(cuts[:-1], cuts[1:])], axis=1)
+    assert np.array_equal(got, oracle.run(drive))
+    mine, theirs = solver.state(), oracle.state()
+    for key in mine:
+        assert np.array_equal(mine[key], theirs[key]), key
+
+
+@pytest.mark.parametrize("tape", [False, True])
+def test_gpu_gradients_of_segments_of_one_step(tape):
+    layout = _box()
+    args = dict(steps=33, precision="fp32")
+    _same(_gradient(layout, segment=1, tape=tape, launched=False, **args), _gradient(layout, segment=33, tape=False, **args))
