@@ -62,6 +62,9 @@ constexpr uint64_t kGraphCells = 1ull << 23;
 constexpr uint32_t kResidentSmem = 216 * 1024;  // shared memory a block of the resident stepper takes at most
 constexpr uint64_t kClusterCells = 1ull << 16;  // (pitched) cells that a cluster's shared memory may take, to try
 constexpr uint64_t kGatheredSteps = 1024;  // steps the probes' cells are gathered over at most (even)
+// The memory their pressures take at most, and the fewest steps worth gathering over: where these do not fit (a plane
+// of more than 8192 receivers of 64 cells; 4096 in double), each step's probes are read by a kernel of their own.
+constexpr uint64_t kGatheredBytes = 32ull << 20, kGatheredLeast = 16;
 
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
@@ -959,8 +962,8 @@ int launch_piece(fdtd_solver *s, const float *d_signal, uint64_t done, uint64_t 
 template <typename T, bool WIDE, bool SCALED, bool COMP>
 int launch_steps(fdtd_solver *s, const float *d_signal, uint64_t steps, double *d_out, uint64_t stride) {
     for (uint64_t done = 0; done < steps;) {
-        const bool gathers = s->probes && s->record_probes && !s->flowing;
-        const uint64_t count = gathers ? std::min<uint64_t>(steps - done, s->gathered_steps) : steps - done;
+        const bool gathered = s->gathered_count && s->record_probes && !s->flowing;
+        const uint64_t count = gathered ? std::min<uint64_t>(steps - done, s->gathered_steps) : steps - done;
         const int rc = launch_piece<T, WIDE, SCALED, COMP>(s, d_signal + done, done, count, d_out + done, stride);
         if (rc != FDTD_OK) return rc;
         done += count;
@@ -1123,6 +1126,11 @@ void choose_columns(const fdtd_solver *s, const std::vector<uint8_t> &types, uin
     if (best > 1) interior_columns(s, types, best, columns);
 }
 
+// Whether the probes' cells are few enough to be gathered over many steps.
+bool gathers(const fdtd_layout *L, uint64_t e) {
+    return L->probe_start[L->probe_count] * e * kGatheredLeast <= kGatheredBytes;
+}
+
 // Whether the grid takes the resident stepper, by the bytes that its steps touch. It saves a step's
 // launches and event waits; the launched kernels, lean ones of many blocks, keep more loads in flight.
 // Measured, us a step, launched (each kind on its stream) and resident, at so many air cells:
@@ -1132,8 +1140,8 @@ void choose_columns(const fdtd_solver *s, const std::vector<uint8_t> &types, uin
 //   double 1.5M 10.9 and 9.8, 2.6M 14.1 and 14.5, 4.3M 23.8 and 22.4, 8.6M 48.0 and 45.3, 10.8M 58.6 and 61.3; with a layer
 //   0.68M 12.6 and 11.5, 1.3M 24.6 and 20.2-23.3, 2.1M 37-44 and 36-45; wide 0.86M 10.9 and 10.5, 1.7M 14.6 and 16.1.
 bool takes_resident(const fdtd_solver *s, const fdtd_layout *L) {
-    if (L->flow_count) return false;
     const uint64_t e = s->precision == FDTD_FP64 ? 8 : 4, MB = 1000 * 1000;
+    if (L->flow_count || !gathers(L, e)) return false;
     const uint64_t a_cell = 2 * e + (s->precision == FDTD_FP32_COMPENSATED ? e : 0);
     const uint64_t touched = a_cell * s->air + 2 * kLayerSlots * e * L->layer_count;
     if (L->layer_count) return touched <= (e == 4 ? 30 : 72) * MB;
@@ -1714,11 +1722,10 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
         const double *pd;
         if ((rc = upload(s, L->probe_weights, pc, &pd))) return rc;
         g.probe_weights = pd;
-        s->gathered_count = (uint32_t)pc;
+        s->gathered_count = gathers(L, e) ? (uint32_t)pc : 0;
     }
-    // The gathered pressures of a piece's steps: 32 MiB of them at most, 16 steps at least.
     const uint64_t a_step = std::max<uint64_t>(1, s->gathered_count) * e;
-    s->gathered_steps = std::min<uint64_t>(kGatheredSteps, std::max<uint64_t>(16, (32ull << 20) / a_step)) / 2 * 2;
+    s->gathered_steps = std::min<uint64_t>(kGatheredSteps, kGatheredBytes / a_step) / 2 * 2;
     if ((rc = zeros(s, a_step * s->gathered_steps, &s->gathered))) return rc;
     s->host_state_start = std::move(state_start);
     return resident ? set_up_resident_kind(s, link_start, s->host_state_start) : FDTD_OK;

@@ -110,3 +110,19 @@ def test_gpu_gradients_of_segments_of_one_step(tape):
     layout = _box()
     args = dict(steps=33, precision="fp32")
     _same(_gradient(layout, segment=1, tape=tape, launched=False, **args), _gradient(layout, segment=33, tape=False, **args))
+
+
+@pytest.mark.parametrize("cells", [1, 523_000, 540_000])
+@pytest.mark.parametrize("launched", [False, True])
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_gpu_records_of_many_receivers(cells, launched, precision):
+    """Gathered over a launch's steps, over sixteen, or (past 524,288 cells, half as many in double) read every step."""
+    layout = _box()
+    times = -(-cells // len(layout["probe_cells"]))
+    drive = np.random.default_rng(6).standard_normal(70).astype(np.float32)
+    solver = B200WaveSolver(_repeated(layout, times), precision=precision)
+    if launched:
+        solver.set_streams(1)
+    assert solver.info().device_bytes < 80e6
+    got = np.concatenate([solver.run(drive[:37]), solver.run(drive[37:])], axis=1)
+    assert np.array_equal(got, np.tile(OracleSolver(layout, precision).run(drive), (times, 1)))
