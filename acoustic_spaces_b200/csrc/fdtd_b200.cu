@@ -527,6 +527,23 @@ int tensor_map(fdtd_solver *s, CUtensorMap *map, void *base, CUtensorMapDataType
     return FDTD_OK;
 }
 
+// The quads that hold interior cells.
+uint64_t interior_quads(const fdtd_solver *s, const std::vector<uint8_t> &types) {
+    uint64_t count = 0;
+    const BulkArgs &bk = s->bulk;
+    if (!s->interior || types.empty()) return count;
+    const uint64_t quads = s->pitch / 4, plane = s->pitch * s->ny;
+    for (uint64_t z = bk.z0; z < bk.z1; ++z)
+        for (uint64_t y = bk.y0; y < bk.y1; ++y) {
+            const uint8_t *row = &types[plane * z + s->pitch * y];
+            uint32_t some = 0;  // (a sum that the compiler takes by vectors)
+            for (uint64_t q = 0; q < quads; ++q)
+                some += row[4 * q] == kInterior || row[4 * q + 1] == kInterior || row[4 * q + 2] == kInterior || row[4 * q + 3] == kInterior;
+            count += some;
+        }
+    return count;
+}
+
 // The columns of quads of the interior, `planes` planes at most each: every run of planes that
 // holds interior cells, from its first, so that a column's first plane holds one.
 void interior_columns(const fdtd_solver *s, const std::vector<uint8_t> &types, uint64_t planes, std::vector<uint2> &columns) {
@@ -535,6 +552,7 @@ void interior_columns(const fdtd_solver *s, const std::vector<uint8_t> &types, u
     if (!s->interior || types.empty()) return;
     const uint64_t quads = s->pitch / 4, plane = s->pitch * s->ny;
     std::vector<uint32_t> masks(quads);
+    columns.reserve((size_t)(s->interior / (4 * planes)));
     for (uint64_t z0 = bk.z0; z0 < bk.z1; z0 += planes)
         for (uint64_t y = bk.y0; y < bk.y1; ++y) {
             std::fill(masks.begin(), masks.end(), 0u);
@@ -1114,8 +1132,7 @@ int dispatch_run(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
 // 7.46, 7.15, 6.52, 6.86, 7.68 and 8.10: the rule takes 3 for both.)
 void choose_columns(const fdtd_solver *s, const std::vector<uint8_t> &types, uint64_t other, uint64_t warps,
                     std::vector<uint2> &columns) {
-    interior_columns(s, types, 1, columns);
-    const uint64_t quads = columns.size();
+    const uint64_t quads = interior_quads(s, types);
     uint64_t best = 1;
     double least = 1e300;
     for (uint64_t planes = 1; planes <= kColumnPlanes; ++planes) {
@@ -1123,7 +1140,7 @@ void choose_columns(const fdtd_solver *s, const std::vector<uint8_t> &types, uin
         const double cost = (double)rounds * ((double)planes + 2.0);
         if (cost < least) least = cost, best = planes;
     }
-    if (best > 1) interior_columns(s, types, best, columns);
+    interior_columns(s, types, best, columns);
 }
 
 // Whether the probes' cells are few enough to be gathered over many steps.
@@ -1439,6 +1456,21 @@ std::vector<uint32_t> layer_lists(fdtd_solver *s, const fdtd_layout *L) {
     return lane_cell;
 }
 
+// A row's first twelve directions packed and, with `links`, its links {weight, offset} from start[row] on, from the
+// slots' tables. (Formed on the host and copied they took 2 of the 21 ms of a set-up with 700,000 links.)
+__global__ void __launch_bounds__(kBlock) row_links_kernel(const Tables g, const uint32_t *start, uint64_t *directions, uint2 *links) {
+    const uint32_t k = blockIdx.x * kBlock + threadIdx.x, K = g.specials;
+    if (k >= K) return;
+    uint64_t packed = 0;
+    for (uint32_t l = 0, n = g.link_count[k]; l < n; ++l) {
+        const uint64_t at = (uint64_t)l * K + k;
+        const uint32_t d = g.link_direction[at];
+        if (l < (uint32_t)kPackedLinks) packed |= (uint64_t)d << (5 * l);
+        if (links) links[start[k] + l] = make_uint2(__float_as_uint(g.link_weight[at]), (uint32_t)g.offset[d]);
+    }
+    directions[k] = packed;
+}
+
 int build(fdtd_solver *s, const fdtd_layout *L) {
     const uint64_t nx = L->nx, ny = L->ny, nz = L->nz, n = nx * ny * nz;
     s->nx = nx, s->ny = ny, s->nz = nz, s->n = n;
@@ -1588,11 +1620,6 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
         g.link_count = u8;
         if ((rc = upload(s, direction.data(), direction.size(), &u8))) return rc;
         g.link_direction = u8;
-        std::vector<uint64_t> packed(K, 0);
-        for (uint64_t k = 0; k < K; ++k)
-            for (uint64_t l = L->link_start[k], n = 0; l < L->link_start[k + 1] && n < kPackedLinks; ++l, ++n)
-                packed[k] |= (uint64_t)L->link_direction[l] << (5 * n);
-        if ((rc = upload(s, packed.data(), K, &g.link_directions))) return rc;
         if ((rc = upload(s, weight.data(), weight.size(), &fp))) return rc;
         g.link_weight = fp;
         // Every row's links axial, in the directions' order, of the axial weight: masks.
@@ -1613,19 +1640,20 @@ int build(fdtd_solver *s, const fdtd_layout *L) {
             if ((rc = upload(s, mask.data(), K, &u8))) return rc;
             g.link_mask = u8;
         }
+        // Each row's packed directions, and the resident stepper's links row by row, from the slots' tables.
+        void *directions, *links = nullptr;
+        if ((rc = zeros(s, sizeof(uint64_t) * K, &directions))) return rc;
+        g.link_directions = static_cast<const uint64_t *>(directions);
         if (resident) {
-            // The resident stepper's links, row by row.
-            std::vector<uint2> links(L->link_count);
-            for (uint64_t l = 0; l < L->link_count; ++l) {
-                uint32_t weight_bits;
-                std::memcpy(&weight_bits, &L->link_weight[l], 4);
-                links[l] = make_uint2(weight_bits, (uint32_t)g.offset[L->link_direction[l]]);
-            }
             link_start.resize(K + 1);
             for (uint64_t k = 0; k <= K; ++k) link_start[k] = (uint32_t)L->link_start[k];
-            if ((rc = upload(s, links.data(), links.size(), &s->row_links))) return rc;
             if ((rc = upload(s, link_start.data(), link_start.size(), &s->link_start))) return rc;
+            if ((rc = zeros(s, sizeof(uint2) * L->link_count, &links))) return rc;
+            s->row_links = static_cast<const uint2 *>(links);
         }
+        if (K) row_links_kernel<<<(uint32_t)((K + kBlock - 1) / kBlock), kBlock, 0, s->stream>>>(
+                g, s->link_start, static_cast<uint64_t *>(directions), static_cast<uint2 *>(links));
+        CUDA_TRY(s, cudaGetLastError());
     }
     if ((rc = upload(s, L->coef_a, K, &fp))) return rc;
     g.coef_a = fp;
@@ -2868,14 +2896,16 @@ int fdtd_create(const fdtd_layout *layout, int precision, int device, fdtd_solve
         cudaGetLastError();
         return set_global(FDTD_ENODEV, "no CUDA device to step the wave grid on");
     }
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, device) != cudaSuccess || prop.major != 10)
+    // (The two attributes alone: the device's whole properties take 2.4 ms to ask for.)
+    int major = 0, sms = 0;
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || major != 10)
         return set_global(FDTD_ENODEV, "the wave stepper is built for sm_100a (B200) only");
     DeviceGuard guard(device);
     fdtd_solver *s = new (std::nothrow) fdtd_solver();
     if (!s) return set_global(FDTD_ENOMEM, "out of host memory");
     s->device = device;
-    s->sms = prop.multiProcessorCount;
+    s->sms = sms;
     s->precision = precision;
     cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking);
