@@ -65,7 +65,7 @@ struct AdjointTables {
     // The matched layer (fdtd.hpp:2242-2264): its cells (pitched), the packed per-axis tables
     // {keep, push, keep_face, push_face} by grid coordinate, each cell's scale with a speed field.
     uint32_t layers, lanes;
-    const uint32_t *layer_cells, *cell_lane;  // (each cell's lane among the forward's quads)
+    const uint32_t *layer_cells, *cell_lane;  // (each cell's lane among the forward's factors; null: its own number)
     const float4 *layer_coef[3];
     const float *layer_scale;
     uint32_t pitch, plane;
@@ -295,7 +295,7 @@ __device__ __forceinline__ void layer_hat_cell(const AdjointTables &t, uint32_t 
         hv[2 * a + 1] = (T)c1.w * hi_hat;
         if (g && traj) {
             const uint64_t M = t.lanes;
-            const T *f = traj + (uint64_t)(6 * a) * M + t.cell_lane[c];
+            const T *f = traj + (uint64_t)(6 * a) * M + (t.cell_lane ? t.cell_lane[c] : c);
             double *gg = g + (uint64_t)(6 * a) * L + c;
             gg[0] += (double)q_hat * (double)f[0];
             gg[(uint64_t)1 * L] += -(double)q_hat * (double)s * (double)f[1 * M];
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(kBlock) layer_pending_kernel(const AdjointTabl
     const uint32_t L = t.layers;
     if (c >= L) return;
     const T s = t.layer_scale ? (T)t.layer_scale[c] : (T)1;
-    const uint32_t a = blockIdx.y, lane = t.cell_lane[c];
+    const uint32_t a = blockIdx.y, lane = t.cell_lane ? t.cell_lane[c] : c;
     const uint64_t M = t.lanes;
     double *gg = g + (uint64_t)(6 * a) * L + c;
     double sum[6];

@@ -258,7 +258,8 @@ struct fdtd_solver {
     // written as level k + record_offset of record_u and record_w; the gradient's recomputation
     // needs no probe records (record_probes false).
     void *record_u = nullptr, *record_w = nullptr;
-    void *record_layer = nullptr;  // the layer's factors of each step (kLayerFactors x layers a step)
+    void *record_layer = nullptr;  // the layer's factors of each step (kLayerFactors x layer_lanes a step)
+    bool record_cells = false;     // (by the layer's cells, kLayerFactors x layers a step)
     uint64_t record_offset = 2;
     bool record_probes = true;
     // The tape (fdtd_set_tape): a run of fdtd_run from rest keeps, for the gradient that follows,
@@ -888,7 +889,8 @@ int launch_piece(fdtd_solver *s, const float *d_signal, uint64_t done, uint64_t 
             f.traj_w = static_cast<T *>(s->record_w) + (at + s->record_offset) * s->states;
         }
         // The matched layer's factors of the step (the gradient's recomputation).
-        if (s->record_layer) f.traj_layer = static_cast<T *>(s->record_layer) + at * kLayerFactors * g.layer_lanes;
+        if (s->record_layer)
+            f.traj_layer = static_cast<T *>(s->record_layer) + at * kLayerFactors * (s->record_cells ? g.layers : g.layer_lanes);
         // The factors of the step along the tables' tangent (a gradient's recomputation, or a taped run).
         if (s->record_tangent) f.traj_tangent = static_cast<T *>(s->record_tangent) + at * s->tangent_factors;
         if (fork) {
@@ -945,7 +947,10 @@ int launch_piece(fdtd_solver *s, const float *d_signal, uint64_t done, uint64_t 
             priority.val.priority = s->layer_priority;
             config.attrs = &priority;
             config.numAttrs = 1;
-            CUDA_TRY(s, cudaLaunchKernelEx(&config, layer_kernel<T, SCALED, COMP>, g, f));
+            if (!COMP && s->record_cells)
+                CUDA_TRY(s, cudaLaunchKernelEx(&config, layer_kernel<T, SCALED, false, true>, g, f));
+            else
+                CUDA_TRY(s, cudaLaunchKernelEx(&config, layer_kernel<T, SCALED, COMP>, g, f));
         }
         if (ev) CUDA_TRY(s, cudaEventRecord(ev[3], layer));
         if (ev) CUDA_TRY(s, cudaEventRecord(ev[4], side));
@@ -1119,7 +1124,8 @@ int dispatch_run(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
     // (A single step is launched: the resident stepper's launch, which loads and stores each block's tables and state,
     // took 14.4 to 20.9 us of one step on 2,000 to 870,000 cells, the launched kernels 12.4 to 16.6; two steps 16 to 27
     // and 20 to 27.)
-    if (s->resident && !s->timing && steps > 1)
+    // (Factors by the layer's cells are the launched kernels' alone.)
+    if (s->resident && !s->timing && steps > 1 && !s->record_cells)
         return s->layers ? launch_resident<T, W, S, C, !W>(s, d_signal, steps, d_out, stride)
                          : launch_resident<T, W, S, C, false>(s, d_signal, steps, d_out, stride);
     return launch_steps<T, W, S, C>(s, d_signal, steps, d_out, stride);
@@ -2360,7 +2366,7 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
     }
     const uint64_t level_bytes = e * s->n_device, state_bytes = e * S;
     // The matched layer: its factors of each step of a segment, and its gradient's sums per cell.
-    const uint64_t Lc = s->layers, lanes = s->tables.layer_lanes;
+    const uint64_t Lc = s->layers, lanes = adj.t.lanes;
     const bool tangent = Lc && s->tangent;  // along a tangent of the tables, in place of the tables
     const bool tables = Lc && s->gradient_tables && !tangent;
     T *traj_layer = nullptr, *waiting = nullptr;
@@ -2450,10 +2456,11 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
     // reverse steps.
     auto recompute = [&](uint64_t count) -> int {
         s->record_u = traj_u, s->record_w = traj_w, s->record_offset = 2, s->record_probes = false;
-        s->record_layer = tables ? traj_layer : nullptr;
+        s->record_layer = tables ? traj_layer : nullptr, s->record_cells = tables && !adj.t.cell_lane;
         s->record_tangent = tangent ? traj_tan : nullptr;
         const int r = dispatch(s, seg_signal, count, d_out, segment);
-        s->record_u = s->record_w = s->record_layer = s->record_tangent = nullptr, s->record_probes = true;
+        s->record_u = s->record_w = s->record_layer = s->record_tangent = nullptr;
+        s->record_cells = false, s->record_probes = true;
         return r;
     };
     // Steps first, first - 1, ... (`count` of them) by the resident reverse stepper, the trajectory's level
@@ -2745,10 +2752,7 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
 // only through the address cudaGetSymbolAddress gives (pool_address).
 constexpr size_t kPoolBytes = FDTD_GRADIENT_STATIC_BYTES;
 constexpr size_t kPoolAlign = 256;
-// A gradient is taken when its buffers by cells fit kPoolBytes. The layer's factors lie by its quads' lanes, of
-// which there are 1.1 to 1.3 a cell in layers of eight cells and up to 4 in layers of one: the pool has room for them.
-constexpr size_t kPoolRoom = 4 * kPoolBytes;
-static __device__ __align__(256) unsigned char g_gradient_pool[kPoolRoom];
+static __device__ __align__(256) unsigned char g_gradient_pool[kPoolBytes];
 
 constexpr size_t pool_round(size_t bytes) { return ((bytes ? bytes : 16) + kPoolAlign - 1) / kPoolAlign * kPoolAlign; }
 
@@ -2774,7 +2778,7 @@ struct StaticPool {
     int take(size_t bytes, void **out, bool zero) {
         *out = nullptr;
         const size_t size = pool_round(bytes);
-        if (used + size > kPoolRoom) return fail(s, FDTD_EINVAL, "the gradient's buffers outgrow the static pool");
+        if (used + size > kPoolBytes) return fail(s, FDTD_EINVAL, "the gradient's buffers outgrow the static pool");
         *out = base + used;
         used += size;
         if (zero) CUDA_TRY(s, cudaMemsetAsync(*out, 0, size, s->stream));
@@ -3147,7 +3151,7 @@ int fdtd_gradient_noalloc(fdtd_solver *s, const float *signal, uint64_t steps, c
     const bool taped = holds_tape(s, signal, steps, segment);
     const uint64_t lanes = s->tables.layer_lanes;
     const size_t need = pool_bytes(s, lists, steps, segment, taped, s->layers, s->layers ? s->n_device : 0);
-    if (need > kPoolBytes || pool_bytes(s, lists, steps, segment, taped, lanes, lanes) > kPoolRoom) {
+    if (need > kPoolBytes) {
         char message[200];
         std::snprintf(message, sizeof message,
                       "the gradient needs %llu bytes of device memory; the static pool holds %llu: fewer steps, a "
@@ -3160,6 +3164,10 @@ int fdtd_gradient_noalloc(fdtd_solver *s, const float *signal, uint64_t steps, c
     StaticPool pool{s, static_cast<char *>(base)};
     AdjointState adj;
     if ((rc = place_adjoint(s, lists, pool, adj)) != FDTD_OK) return rc;
+    // The layer's factors lie by its quads' lanes, 1.1 to 1.3 a cell in layers of eight cells, up to 16 where each cell
+    // lies alone: where those do not fit, by the layer's cells.
+    if (pool_bytes(s, lists, steps, segment, taped, lanes, lanes) > kPoolBytes)
+        adj.t.lanes = (uint32_t)s->layers, adj.t.cell_lane = nullptr;
     double *grads[5] = {grad_coef_b, grad_coef_inv, grad_now, grad_before, grad_gain};
     // (No graphs: instantiating one allocates.)
     return s->precision == FDTD_FP64 ? gradient<double>(s, adj, pool, signal, steps, dloss_dy, segment, grads, false)

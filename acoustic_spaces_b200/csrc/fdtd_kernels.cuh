@@ -846,7 +846,8 @@ __device__ __forceinline__ void store_layer(T *now, const uint64_t lanes, const 
 
 // A step of a quad's state (in place) and its new pressures. (Lanes outside the layer are worked out
 // too, and stored nowhere.)
-template <typename T, bool SCALED, bool COMP, bool STREAM>
+// CELLS: the tables' factors go to their cells' numbers in place of the quad's lanes.
+template <typename T, bool SCALED, bool COMP, bool STREAM, bool CELLS = false>
 __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, const float4 *const (&coef)[3], const uint32_t q,
                                            const uint4 d, LayerState<T> &s) {
     const uint32_t mask = d.w & 15u, i = d.x;
@@ -867,7 +868,14 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
         for (int j = 0; j < (a == 0 ? 5 : 2); ++j) c[j] = a == 0 ? coef[0][(j % 4) * g.x_quads + x / 4 + j / 4] : coef[a][at + j];
         // The step's factors of the tables' gradient, a quad each (a cell at a time they took 13.5 of the
         // 22 us of a recorded step of 0.32M layer cells).
-        T *factors = f.traj_layer ? f.traj_layer + (uint64_t)(6 * a) * g.layer_lanes + 4 * (uint64_t)q : nullptr;
+        const uint64_t stride = CELLS ? g.layers : g.layer_lanes;
+        T *factors = f.traj_layer ? f.traj_layer + (uint64_t)(6 * a) * stride + (CELLS ? 0 : 4 * (uint64_t)q) : nullptr;
+        auto record = [&](int k, const Quad<T> &v) {
+            if (!CELLS) return store_quad<true>(factors + k * stride, v);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (mask & (1u << j)) factors[k * stride + g.lane_cell[4 * (uint64_t)q + j]] = v.v[j];
+        };
         if (factors) {
             Quad<T> up, down;
 #pragma unroll
@@ -875,11 +883,7 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
                 up.v[j] = (a == 0 ? (j == 3 ? right : h.v[j + 1]) : (a == 1 ? yp.v[j] : zp.v[j])) - h.v[j];
                 down.v[j] = h.v[j] - (a == 0 ? (j == 0 ? left : h.v[j - 1]) : (a == 1 ? ym.v[j] : zm.v[j]));
             }
-            store_quad<true>(factors, s.part[a]);
-            store_quad<true>(factors + 2 * (uint64_t)g.layer_lanes, s.hi[a]);
-            store_quad<true>(factors + 3 * (uint64_t)g.layer_lanes, up);
-            store_quad<true>(factors + 4 * (uint64_t)g.layer_lanes, s.lo[a]);
-            store_quad<true>(factors + 5 * (uint64_t)g.layer_lanes, down);
+            record(0, s.part[a]), record(2, s.hi[a]), record(3, up), record(4, s.lo[a]), record(5, down);
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -918,7 +922,7 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
             }
             s.lo[a].v[j] = below, s.hi[a].v[j] = above;
         }
-        if (factors) store_quad<true>(factors + g.layer_lanes, rise);
+        if (factors) record(1, rise);
     }
     if (COMP) {
         Quad<T> next;
@@ -931,20 +935,20 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
     }
 }
 
-template <typename T, bool SCALED, bool COMP, bool STREAM = true>
+template <typename T, bool SCALED, bool COMP, bool CELLS, bool STREAM = true>
 __device__ __forceinline__ void layer_quad(const Tables &g, const Fields<T> &f, const uint32_t q, const uint4 d) {
     if (!(d.w & 15u)) return;  // (it only keeps a face for the quads above)
     LayerState<T> s;
     load_layer(f.cell_old, g.layer_lanes, q, d, s);
     const float4 *const coef[3] = {g.layer_coef_x, g.layer_coef[1], g.layer_coef[2]};
-    step_layer<T, SCALED, COMP, STREAM>(g, f, coef, q, d, s);
+    step_layer<T, SCALED, COMP, STREAM, CELLS>(g, f, coef, q, d, s);
     store_layer<STREAM>(f.cell_new, g.layer_lanes, q, d, s);
 }
 
 // A grid of a few blocks an SM (the sweep's blocks keep their places beside it), each thread taking
 // quads q, q + the grid's threads, ...; the next quad's entry is loaded while this one's loads are
 // in flight, so that a quad costs one round trip to memory rather than two.
-template <typename T, bool SCALED, bool COMP = false>
+template <typename T, bool SCALED, bool COMP = false, bool CELLS = false>
 __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? 4 : 3) layer_kernel(const Tables g, const Fields<T> f) {
     const uint32_t n = g.layer_quads;
     const uint32_t step = gridDim.x * kBlock;
@@ -954,7 +958,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? 4 : 3) layer_kernel(c
     for (; q < n; q += step) {
         const uint4 entry = next;
         if (q + step < n) next = __ldg(g.layer_quad + q + step);
-        layer_quad<T, SCALED, COMP>(g, f, q, entry);
+        layer_quad<T, SCALED, COMP, CELLS>(g, f, q, entry);
     }
 }
 

@@ -383,8 +383,7 @@ int fdtd_set_launch(fdtd_solver *solver, int layer_per_sm, int special_per_sm);
 int fdtd_set_coefficients(fdtd_solver *solver, const float *coef_b, const float *coef_inv, const float *branch_now,
                           const float *branch_before, const float *branch_gain);
 
-/* Bytes of the static device pool of fdtd_gradient_noalloc: 16 MiB, in 64 MiB (the matched layer's
- * buffers are padded to whole quads of cells) held on every device the
+/* Bytes of the static device pool of fdtd_gradient_noalloc: 16 MiB, held on every device the
    library runs on until the process exits. */
 #define FDTD_GRADIENT_STATIC_BYTES (16ull << 20)
 
