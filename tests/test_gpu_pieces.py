@@ -126,3 +126,23 @@ def test_gpu_records_of_many_receivers(cells, launched, precision):
     assert solver.info().device_bytes < 80e6
     got = np.concatenate([solver.run(drive[:37]), solver.run(drive[37:])], axis=1)
     assert np.array_equal(got, np.tile(OracleSolver(layout, precision).run(drive), (times, 1)))
+
+
+@pytest.mark.parametrize("speed", [None, 0.97])
+def test_gpu_rows_that_shared_memory_does_not_hold(speed):
+    """A 7.5M-cell room in double, 1550 rows a block of 5 branch states each: the resident stepper reads its rows' tables
+    from memory."""
+    rng = np.random.default_rng(7)
+    shape = np.array([200, 195, 192])
+    walls = [layouts.Material(0.05, np.vstack([layouts.resonant_branch(0.1, 2.0, f, 5000.0) for f in rng.uniform(40, 200, 5)]))
+             for _ in range(6)]  # fmt: skip
+    grid = layouts.Grid(-0.2 * np.ones(3), 0.1, tuple(int(v) + 4 for v in shape))
+    points = [np.array([0.35, 0.35, 0.35]), np.array([0.75, 0.45, 0.35])]
+    layout = layouts.cell_face_layout(layouts.shoebox(0.1 * shape, walls), grid, points[0], points[1:], speed=speed,
+                                      rate=5000.0).layout  # fmt: skip
+    drive = rng.standard_normal(14).astype(np.float32)
+    solver, oracle = B200WaveSolver(layout, precision="fp64", autotune=False), OracleSolver(layout, "fp64")
+    assert np.array_equal(np.concatenate([solver.run(drive[:9]), solver.run(drive[9:])], axis=1), oracle.run(drive))
+    mine, theirs = solver.state(), oracle.state()
+    for key in mine:
+        assert np.array_equal(mine[key], theirs[key]), key
