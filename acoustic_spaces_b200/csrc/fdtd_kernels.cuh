@@ -844,9 +844,21 @@ __device__ __forceinline__ void store_layer(T *now, const uint64_t lanes, const 
     if (keep_z) store_cells<STREAM>(now + 5 * lanes + 4 * (uint64_t)d.z, s.lo[2], keep_z);
 }
 
+// A quad's factor f of the tables' gradient: to its lanes, or CELLS to its layer cells' numbers.
+template <bool CELLS, typename T>
+__device__ __forceinline__ void store_factor(const Tables &g, T *factors, const uint32_t f, const Quad<T> &v, const uint32_t q,
+                                             const uint32_t mask) {
+    if constexpr (CELLS) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (mask & (1u << j)) factors[(uint64_t)f * g.layers + g.lane_cell[4 * (uint64_t)q + j]] = v.v[j];
+    } else {
+        store_quad<true>(factors + f * (uint64_t)g.layer_lanes, v);
+    }
+}
+
 // A step of a quad's state (in place) and its new pressures. (Lanes outside the layer are worked out
 // too, and stored nowhere.)
-// CELLS: the tables' factors go to their cells' numbers in place of the quad's lanes.
 template <typename T, bool SCALED, bool COMP, bool STREAM, bool CELLS = false>
 __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, const float4 *const (&coef)[3], const uint32_t q,
                                            const uint4 d, LayerState<T> &s) {
@@ -868,14 +880,7 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
         for (int j = 0; j < (a == 0 ? 5 : 2); ++j) c[j] = a == 0 ? coef[0][(j % 4) * g.x_quads + x / 4 + j / 4] : coef[a][at + j];
         // The step's factors of the tables' gradient, a quad each (a cell at a time they took 13.5 of the
         // 22 us of a recorded step of 0.32M layer cells).
-        const uint64_t stride = CELLS ? g.layers : g.layer_lanes;
-        T *factors = f.traj_layer ? f.traj_layer + (uint64_t)(6 * a) * stride + (CELLS ? 0 : 4 * (uint64_t)q) : nullptr;
-        auto record = [&](int k, const Quad<T> &v) {
-            if (!CELLS) return store_quad<true>(factors + k * stride, v);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (mask & (1u << j)) factors[k * stride + g.lane_cell[4 * (uint64_t)q + j]] = v.v[j];
-        };
+        T *factors = f.traj_layer ? f.traj_layer + (uint64_t)(6 * a) * (CELLS ? g.layers : g.layer_lanes) + (CELLS ? 0 : 4 * (uint64_t)q) : nullptr;
         if (factors) {
             Quad<T> up, down;
 #pragma unroll
@@ -883,7 +888,11 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
                 up.v[j] = (a == 0 ? (j == 3 ? right : h.v[j + 1]) : (a == 1 ? yp.v[j] : zp.v[j])) - h.v[j];
                 down.v[j] = h.v[j] - (a == 0 ? (j == 0 ? left : h.v[j - 1]) : (a == 1 ? ym.v[j] : zm.v[j]));
             }
-            record(0, s.part[a]), record(2, s.hi[a]), record(3, up), record(4, s.lo[a]), record(5, down);
+            store_factor<CELLS>(g, factors, 0, s.part[a], q, mask);
+            store_factor<CELLS>(g, factors, 2, s.hi[a], q, mask);
+            store_factor<CELLS>(g, factors, 3, up, q, mask);
+            store_factor<CELLS>(g, factors, 4, s.lo[a], q, mask);
+            store_factor<CELLS>(g, factors, 5, down, q, mask);
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -922,7 +931,7 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
             }
             s.lo[a].v[j] = below, s.hi[a].v[j] = above;
         }
-        if (factors) record(1, rise);
+        if (factors) store_factor<CELLS>(g, factors, 1, rise, q, mask);
     }
     if (COMP) {
         Quad<T> next;
