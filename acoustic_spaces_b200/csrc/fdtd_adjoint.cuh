@@ -65,7 +65,7 @@ struct AdjointTables {
     // The matched layer (fdtd.hpp:2242-2264): its cells (pitched), the packed per-axis tables
     // {keep, push, keep_face, push_face} by grid coordinate, each cell's scale with a speed field.
     uint32_t layers, lanes;
-    const uint32_t *layer_cells, *cell_lane;  // (each cell's lane among the forward's factors; null: its own number)
+    const uint32_t *layer_cells, *cell_lane;  // (each cell's lane among the forward's quads; null: factors by cells)
     const float4 *layer_coef[3];
     const float *layer_scale;
     uint32_t pitch, plane;
@@ -263,7 +263,9 @@ __device__ __forceinline__ double tangent_products(const AdjointTables &t, uint3
     return sum;
 }
 
-template <typename T>
+// CELLS: the factors lie by the cells' own numbers. (Asked at run time, of a null table, it took the kernel in double from
+// 56 to 66 registers and its 8 blocks an SM to 7: 132 -> 205 us on 0.9M layer cells.)
+template <typename T, bool CELLS = false>
 __device__ __forceinline__ void layer_hat_cell(const AdjointTables &t, uint32_t c, uint32_t i, T lam, T *carried, T *hat,
                                                const T *traj, double *g, T *pending, const T *tangent = nullptr) {
     const uint32_t L = t.layers;
@@ -295,7 +297,7 @@ __device__ __forceinline__ void layer_hat_cell(const AdjointTables &t, uint32_t 
         hv[2 * a + 1] = (T)c1.w * hi_hat;
         if (g && traj) {
             const uint64_t M = t.lanes;
-            const T *f = traj + (uint64_t)(6 * a) * M + (t.cell_lane ? t.cell_lane[c] : c);
+            const T *f = traj + (uint64_t)(6 * a) * M + (CELLS ? c : t.cell_lane[c]);
             double *gg = g + (uint64_t)(6 * a) * L + c;
             gg[0] += (double)q_hat * (double)f[0];
             gg[(uint64_t)1 * L] += -(double)q_hat * (double)s * (double)f[1 * M];
@@ -333,14 +335,14 @@ __device__ __forceinline__ void layer_hat_cell(const AdjointTables &t, uint32_t 
 // steps' products are added in turn, one read and write of a cell's eighteen double sums for all of
 // them (their 288 bytes a cell are most of what a step of the tables' gradient moves). A row of blocks an
 // axis.
-template <typename T>
+template <typename T, bool CELLS = false>
 __global__ void __launch_bounds__(kBlock) layer_pending_kernel(const AdjointTables t, const T *waiting, uint32_t steps,
                                                                const T *traj, double *g) {
     const uint32_t c = blockIdx.x * kBlock + threadIdx.x;
     const uint32_t L = t.layers;
     if (c >= L) return;
     const T s = t.layer_scale ? (T)t.layer_scale[c] : (T)1;
-    const uint32_t a = blockIdx.y, lane = t.cell_lane ? t.cell_lane[c] : c;
+    const uint32_t a = blockIdx.y, lane = CELLS ? c : t.cell_lane[c];
     const uint64_t M = t.lanes;
     double *gg = g + (uint64_t)(6 * a) * L + c;
     double sum[6];
@@ -477,7 +479,7 @@ struct LayerNext {
 // s lam), the rows linking to it, the layer's terms and the probes' terms (a layer cell's update
 // reads no level before the last, so no level two steps on enters); then, from it, the cell's hats
 // of the step before (layer_hat_cell).
-template <typename T>
+template <typename T, bool CELLS = false>
 __device__ __forceinline__ void layer_adjoint_cell(const AdjointTables &t, uint32_t c, const T *lam_next, const T *tilde,
                                                    const T *hat, T *lam_out, const double *dloss, uint64_t stride,
                                                    uint64_t step, const LayerNext<T> &next) {
@@ -500,7 +502,7 @@ __device__ __forceinline__ void layer_adjoint_cell(const AdjointTables &t, uint3
     }
     lam_out[i] = value;
     const T *tangent = next.tangent_base && !next.pending ? *next.tangent_base + next.tangent_offset : nullptr;
-    layer_hat_cell<T>(t, c, i, value, next.carried, next.hat, next.traj, next.g, next.pending, tangent);
+    layer_hat_cell<T, CELLS>(t, c, i, value, next.carried, next.hat, next.traj, next.g, next.pending, tangent);
 }
 
 // One launch of the special rows' adjoint (the rows special_order[begin .. end), on the first
@@ -515,7 +517,7 @@ struct RowsPart {
     __host__ __device__ uint32_t blocks() const { return special_blocks + corrected_blocks + layer_blocks; }
 };
 
-template <typename T>
+template <typename T, bool CELLS = false>
 __global__ void __launch_bounds__(kBlock) rows_adjoint_kernel(const AdjointTables t, const RowsPart part,
                                                               const T *lam_next, const T *om_next, const T *tilde,
                                                               const T *hat, T *lam_out, T *om_out, const T *traj_u,
@@ -535,7 +537,7 @@ __global__ void __launch_bounds__(kBlock) rows_adjoint_kernel(const AdjointTable
         if (e < part.corrected_end)
             correct_cell<T>(t, t.corrected_order[e], lam_next, tilde, hat, lam_out, dloss, stride, step);
     } else {
-        layer_adjoint_cell<T>(t, (b - part.special_blocks - part.corrected_blocks) * kBlock + threadIdx.x, lam_next,
+        layer_adjoint_cell<T, CELLS>(t, (b - part.special_blocks - part.corrected_blocks) * kBlock + threadIdx.x, lam_next,
                               tilde, hat, lam_out, dloss, stride, step, next);
     }
     }

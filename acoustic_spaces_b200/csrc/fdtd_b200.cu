@@ -2542,9 +2542,10 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
                     t, far, lam_next, om_next, tilde, hat, lam_out, om_out, traj_u, traj_w, (uint32_t)m, g[1], g[0],
                     g[2], g[3], g[4], tilde_out, seg_dloss, segment, m, next);
             if (layer_blocks) {
-                rows_adjoint_kernel<T><<<near_grid, kBlock, 0, s->layer_stream>>>(t, near, lam_next, om_next, tilde, hat, lam_out, om_out,
-                                                            traj_u, traj_w, (uint32_t)m, g[1], g[0], g[2], g[3], g[4],
-                                                            tilde_out, seg_dloss, segment, m, next);
+                auto kernel = t.cell_lane ? rows_adjoint_kernel<T> : rows_adjoint_kernel<T, true>;
+                kernel<<<near_grid, kBlock, 0, s->layer_stream>>>(t, near, lam_next, om_next, tilde, hat, lam_out, om_out,
+                                                                  traj_u, traj_w, (uint32_t)m, g[1], g[0], g[2], g[3], g[4],
+                                                                  tilde_out, seg_dloss, segment, m, next);
                 CUDA_TRY(s, cudaEventRecord(s->joined[2], s->layer_stream));
             }
             CUDA_TRY(s, cudaEventRecord(s->joined[1], s->side));
@@ -2682,7 +2683,8 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
         // The layer's products of this segment's last step, whose Q^, L^, H^ the segment after
         // left waiting: its factors are recorded now.
         if (tables && k + 1 < segments) {
-            layer_pending_kernel<T><<<dim3(layer_blocks, 3), kBlock, 0, s->stream>>>(
+            auto kernel = t.cell_lane ? layer_pending_kernel<T> : layer_pending_kernel<T, true>;
+            kernel<<<dim3(layer_blocks, 3), kBlock, 0, s->stream>>>(
                 t, static_cast<const T *>(adj.pending), 1, traj_layer + (count - 1) * kLayerFactors * lanes, g_layer);
             CUDA_TRY(s, cudaGetLastError());
         }
