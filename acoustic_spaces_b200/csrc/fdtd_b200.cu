@@ -947,10 +947,12 @@ int launch_piece(fdtd_solver *s, const float *d_signal, uint64_t done, uint64_t 
             priority.val.priority = s->layer_priority;
             config.attrs = &priority;
             config.numAttrs = 1;
-            if (!COMP && s->record_cells)
-                CUDA_TRY(s, cudaLaunchKernelEx(&config, layer_kernel<T, SCALED, false, true>, g, f));
-            else
-                CUDA_TRY(s, cudaLaunchKernelEx(&config, layer_kernel<T, SCALED, COMP>, g, f));
+            auto kernel = layer_kernel<T, SCALED, COMP>;
+            if (!COMP && f.traj_tangent)
+                kernel = layer_kernel<T, SCALED, false, kTangent>;
+            else if (!COMP && f.traj_layer)
+                kernel = s->record_cells ? layer_kernel<T, SCALED, false, kCells> : layer_kernel<T, SCALED, false, kLanes>;
+            CUDA_TRY(s, cudaLaunchKernelEx(&config, kernel, g, f));
         }
         if (ev) CUDA_TRY(s, cudaEventRecord(ev[3], layer));
         if (ev) CUDA_TRY(s, cudaEventRecord(ev[4], side));

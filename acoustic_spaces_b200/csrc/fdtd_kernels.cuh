@@ -844,6 +844,11 @@ __device__ __forceinline__ void store_layer(T *now, const uint64_t lanes, const 
     if (keep_z) store_cells<STREAM>(now + 5 * lanes + 4 * (uint64_t)d.z, s.lo[2], keep_z);
 }
 
+// What a step of the layer records: whatever the fields ask for (the resident stepper), nothing, the factors of the
+// tables' gradient by lanes or by cells, or those along a tangent. (The launched kernels are apart, as the code of one
+// takes registers of the others.)
+enum Record { kAsked, kNothing, kLanes, kCells, kTangent };
+
 // A quad's factor f of the tables' gradient: to its lanes, or CELLS to its layer cells' numbers.
 template <bool CELLS, typename T>
 __device__ __forceinline__ void store_factor(const Tables &g, T *factors, const uint32_t f, const Quad<T> &v, const uint32_t q,
@@ -859,7 +864,7 @@ __device__ __forceinline__ void store_factor(const Tables &g, T *factors, const 
 
 // A step of a quad's state (in place) and its new pressures. (Lanes outside the layer are worked out
 // too, and stored nowhere.)
-template <typename T, bool SCALED, bool COMP, bool STREAM, bool CELLS = false>
+template <typename T, bool SCALED, bool COMP, bool STREAM, Record RECORD = kAsked>
 __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, const float4 *const (&coef)[3], const uint32_t q,
                                            const uint4 d, LayerState<T> &s) {
     const uint32_t mask = d.w & 15u, i = d.x;
@@ -870,7 +875,17 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
     const T left = b[i - 1], right = b[i + 4];
     const uint32_t z = g.by_plane(i), r = i - z * g.plane, y = g.by_pitch(r), x = r - y * g.pitch;
     const Quad<T> sc = scales<T, SCALED>(g.lane_scale, 4 * q);
-    const bool recording = f.traj_tangent;
+    constexpr bool CELLS = RECORD == kCells;
+    const bool recording = RECORD == kAsked ? f.traj_tangent != nullptr : RECORD == kTangent;
+    uint4 cells = make_uint4(0, 0, 0, 0);
+    uint32_t tangent_axes = 0;  // the cells' axes, a byte each
+    if (RECORD == kTangent) {
+        cells = *reinterpret_cast<const uint4 *>(g.lane_cell + 4 * (uint64_t)q);
+        if (mask & 1u) tangent_axes |= g.tangent_axes[cells.x];
+        if (mask & 2u) tangent_axes |= (uint32_t)g.tangent_axes[cells.y] << 8;
+        if (mask & 4u) tangent_axes |= (uint32_t)g.tangent_axes[cells.z] << 16;
+        if (mask & 8u) tangent_axes |= (uint32_t)g.tangent_axes[cells.w] << 24;
+    }
     Quad<T> total{}, rise;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -880,7 +895,8 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
         for (int j = 0; j < (a == 0 ? 5 : 2); ++j) c[j] = a == 0 ? coef[0][(j % 4) * g.x_quads + x / 4 + j / 4] : coef[a][at + j];
         // The step's factors of the tables' gradient, a quad each (a cell at a time they took 13.5 of the
         // 22 us of a recorded step of 0.32M layer cells).
-        T *factors = f.traj_layer ? f.traj_layer + (uint64_t)(6 * a) * (CELLS ? g.layers : g.layer_lanes) + (CELLS ? 0 : 4 * (uint64_t)q) : nullptr;
+        constexpr bool kTables = RECORD == kAsked || RECORD == kLanes || RECORD == kCells;
+        T *factors = kTables && f.traj_layer ? f.traj_layer + (uint64_t)(6 * a) * (CELLS ? g.layers : g.layer_lanes) + (CELLS ? 0 : 4 * (uint64_t)q) : nullptr;
         if (factors) {
             Quad<T> up, down;
 #pragma unroll
@@ -904,8 +920,9 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
             const T below = (T)c0.z * old_below - (T)c0.w * (here - lo);
             const T above = (T)c1.z * old_above - (T)c1.w * (hi - here);
             if (recording && (mask & (1u << j))) {
-                const uint32_t cell = g.lane_cell[4 * (uint64_t)q + j];
-                const uint32_t axes = g.tangent_axes[cell];
+                const uint32_t own = j == 0 ? cells.x : (j == 1 ? cells.y : (j == 2 ? cells.z : cells.w));
+                const uint32_t cell = RECORD == kTangent ? own : g.lane_cell[4 * (uint64_t)q + j];
+                const uint32_t axes = RECORD == kTangent ? tangent_axes >> (8 * j) : g.tangent_axes[cell];
                 if (axes & (1u << a)) {
                     // The step's factors along the tangent: its products with the adjoints of the new
                     // part and faces give the gradient's step (fdtd_adjoint.cuh), in double.
@@ -944,20 +961,20 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
     }
 }
 
-template <typename T, bool SCALED, bool COMP, bool CELLS, bool STREAM = true>
+template <typename T, bool SCALED, bool COMP, Record RECORD, bool STREAM = true>
 __device__ __forceinline__ void layer_quad(const Tables &g, const Fields<T> &f, const uint32_t q, const uint4 d) {
     if (!(d.w & 15u)) return;  // (it only keeps a face for the quads above)
     LayerState<T> s;
     load_layer(f.cell_old, g.layer_lanes, q, d, s);
     const float4 *const coef[3] = {g.layer_coef_x, g.layer_coef[1], g.layer_coef[2]};
-    step_layer<T, SCALED, COMP, STREAM, CELLS>(g, f, coef, q, d, s);
+    step_layer<T, SCALED, COMP, STREAM, RECORD>(g, f, coef, q, d, s);
     store_layer<STREAM>(f.cell_new, g.layer_lanes, q, d, s);
 }
 
 // A grid of a few blocks an SM (the sweep's blocks keep their places beside it), each thread taking
 // quads q, q + the grid's threads, ...; the next quad's entry is loaded while this one's loads are
 // in flight, so that a quad costs one round trip to memory rather than two.
-template <typename T, bool SCALED, bool COMP = false, bool CELLS = false>
+template <typename T, bool SCALED, bool COMP = false, Record RECORD = kNothing>
 __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? 4 : 3) layer_kernel(const Tables g, const Fields<T> f) {
     const uint32_t n = g.layer_quads;
     const uint32_t step = gridDim.x * kBlock;
@@ -967,7 +984,7 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? 4 : 3) layer_kernel(c
     for (; q < n; q += step) {
         const uint4 entry = next;
         if (q + step < n) next = __ldg(g.layer_quad + q + step);
-        layer_quad<T, SCALED, COMP, CELLS>(g, f, q, entry);
+        layer_quad<T, SCALED, COMP, RECORD>(g, f, q, entry);
     }
 }
 
