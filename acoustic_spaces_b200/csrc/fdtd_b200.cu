@@ -1081,8 +1081,7 @@ int launch_resident(fdtd_solver *s, const float *d_signal, uint64_t steps, doubl
             a.traj_w = static_cast<T *>(s->record_w) + (done + s->record_offset) * s->states;
         }
         if (s->record_layer) a.traj_layer = static_cast<T *>(s->record_layer) + done * kLayerFactors * s->tables.layer_lanes;
-        if (s->record_tangent) a.traj_tangent = static_cast<T *>(s->record_tangent) + done * s->tangent_factors;
-        a.states = (uint32_t)s->states, a.tangent_factors = (uint32_t)s->tangent_factors;
+        a.states = (uint32_t)s->states;
         a.steps = (uint32_t)count;
         a.clustered = s->resident_clustered ? 1 : 0;
         a.arrived = s->arrived, a.error = s->d_error;
@@ -1126,8 +1125,8 @@ int dispatch_run(fdtd_solver *s, const float *d_signal, uint64_t steps, double *
     // (A single step is launched: the resident stepper's launch, which loads and stores each block's tables and state,
     // took 14.4 to 20.9 us of one step on 2,000 to 870,000 cells, the launched kernels 12.4 to 16.6; two steps 16 to 27
     // and 20 to 27.)
-    // (Factors by the layer's cells are the launched kernels' alone.)
-    if (s->resident && !s->timing && steps > 1 && !s->record_cells)
+    // (Factors by the layer's cells are the launched kernels' alone; those along a tangent they record sooner.)
+    if (s->resident && !s->timing && steps > 1 && !s->record_cells && !s->record_tangent)
         return s->layers ? launch_resident<T, W, S, C, !W>(s, d_signal, steps, d_out, stride)
                          : launch_resident<T, W, S, C, false>(s, d_signal, steps, d_out, stride);
     return launch_steps<T, W, S, C>(s, d_signal, steps, d_out, stride);
@@ -2593,7 +2592,7 @@ int gradient(fdtd_solver *s, const AdjointState &adj, Pool &scratch, const float
     }
     auto run = [&](int which, int key, auto &&body, uint64_t count) -> int {
         // (The resident stepper's recomputation is a launch or two: nothing to capture.)
-        if (!graphs || count != segment || segments == 1 || (which == 0 ? s->resident && !s->timing : resident)) return body(count);
+        if (!graphs || count != segment || segments == 1 || (which == 0 ? s->resident && !s->timing && !tangent : resident)) return body(count);
         cudaGraphExec_t &exec = s->grad_graph[which][key];
         if (!exec) {
             const bool timing = s->timing;
@@ -2976,7 +2975,6 @@ int fdtd_run(fdtd_solver *s, const float *signal, uint64_t steps, double *out) {
     // Pinned host staging for a piece of the run (the drive and the probes' records), grown on
     // demand; the device side is the handle's chunk buffers, chunk_steps steps at a time.
     const uint64_t P = std::max<uint64_t>(1, s->probes);
-    const bool resident = s->resident && !s->timing;  // (its chunks are no captured graphs)
     const uint64_t piece = std::min<uint64_t>(steps, std::max<uint64_t>(s->chunk_steps, (64ull << 20) / (8 * P)));
     if (s->stage_steps < piece) {
         if (s->stage_signal) cudaFreeHost(s->stage_signal);
@@ -3015,6 +3013,7 @@ int fdtd_run(fdtd_solver *s, const float *signal, uint64_t steps, double *out) {
                     e * (K + S) * (steps + 2) + tangent_bytes <= budget;
     }
     const bool keep_tangent = keep_traj && s->layers && s->tangent;
+    const bool resident = s->resident && !s->timing && !keep_tangent;  // (its chunks are no captured graphs)
     if (keep_traj) {
         int r;
         if (s->tape_levels < steps + 2) {
@@ -3668,7 +3667,7 @@ int fdtd_set_layer_tangent(fdtd_solver *s, const double *tangent, uint64_t count
     s->tangent_device.clear();
     Tables &g = s->tables;
     for (int a = 0; a < 3; ++a) g.tangent_centre[a] = g.tangent_face[a] = nullptr;
-    g.tangent_axes = nullptr, g.tangent_start = nullptr;
+    g.tangent_axes = nullptr, g.tangent_start = nullptr, g.quad_tangent_axes = nullptr, g.quad_tangent_start = nullptr;
     s->tangent = false, s->tangent_factors = 0, s->tangent_valid = false;
     s->tape_valid = false;
     Kept{s}.drop_graphs();
@@ -3739,6 +3738,18 @@ int fdtd_set_layer_tangent(fdtd_solver *s, const double *tangent, uint64_t count
     if ((rc = upload(s, start.data(), Lc, &ps))) return rc;
     s->tangent_device.push_back(const_cast<uint32_t *>(ps));
     g.tangent_axes = pa, g.tangent_start = ps;
+    std::vector<uint32_t> quad_axes(s->layer_quads.size(), 0);
+    std::vector<uint4> quad_start(s->layer_quads.size(), make_uint4(0, 0, 0, 0));
+    for (uint64_t c = 0; c < Lc; ++c) {
+        const uint32_t lane = s->layer_lane[c], j = lane % 4;
+        uint4 &first = quad_start[lane / 4];
+        (j == 0 ? first.x : (j == 1 ? first.y : (j == 2 ? first.z : first.w))) = start[c];
+        quad_axes[lane / 4] |= (uint32_t)axes[c] << (8 * j);
+    }
+    if ((rc = upload(s, quad_axes.data(), quad_axes.size(), &g.quad_tangent_axes))) return rc;
+    s->tangent_device.push_back(const_cast<uint32_t *>(g.quad_tangent_axes));
+    if ((rc = upload(s, quad_start.data(), quad_start.size(), &g.quad_tangent_start))) return rc;
+    s->tangent_device.push_back(const_cast<uint4 *>(g.quad_tangent_start));
     if (old_factors != factors) drop_tape();
     s->tangent_factors = factors;
     s->tangent = true;

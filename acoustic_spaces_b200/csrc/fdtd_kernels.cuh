@@ -554,6 +554,8 @@ struct Tables {
     const double2 *tangent_centre[3], *tangent_face[3];
     const uint8_t *tangent_axes;
     const uint32_t *tangent_start;
+    const uint32_t *quad_tangent_axes;  // the same by the layer's quads: their four cells' axes, a byte each
+    const uint4 *quad_tangent_start;
     // Probes (fdtd.hpp:3525-3533).
     uint32_t probes;
     const uint32_t *probe_start, *probe_cells;
@@ -844,9 +846,9 @@ __device__ __forceinline__ void store_layer(T *now, const uint64_t lanes, const 
     if (keep_z) store_cells<STREAM>(now + 5 * lanes + 4 * (uint64_t)d.z, s.lo[2], keep_z);
 }
 
-// What a step of the layer records: whatever the fields ask for (the resident stepper), nothing, the factors of the
-// tables' gradient by lanes or by cells, or those along a tangent. (The launched kernels are apart, as the code of one
-// takes registers of the others.)
+// What a step of the layer records: nothing, the factors of the tables' gradient by lanes or by cells, or those along a
+// tangent; or those by lanes if the fields ask for them (the resident stepper). (The launched kernels are apart, as the
+// code of one takes registers of the others.)
 enum Record { kAsked, kNothing, kLanes, kCells, kTangent };
 
 // A quad's factor f of the tables' gradient: to its lanes, or CELLS to its layer cells' numbers.
@@ -876,16 +878,9 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
     const uint32_t z = g.by_plane(i), r = i - z * g.plane, y = g.by_pitch(r), x = r - y * g.pitch;
     const Quad<T> sc = scales<T, SCALED>(g.lane_scale, 4 * q);
     constexpr bool CELLS = RECORD == kCells;
-    const bool recording = RECORD == kAsked ? f.traj_tangent != nullptr : RECORD == kTangent;
-    uint4 cells = make_uint4(0, 0, 0, 0);
-    uint32_t tangent_axes = 0;  // the cells' axes, a byte each
-    if (RECORD == kTangent) {
-        cells = *reinterpret_cast<const uint4 *>(g.lane_cell + 4 * (uint64_t)q);
-        if (mask & 1u) tangent_axes |= g.tangent_axes[cells.x];
-        if (mask & 2u) tangent_axes |= (uint32_t)g.tangent_axes[cells.y] << 8;
-        if (mask & 4u) tangent_axes |= (uint32_t)g.tangent_axes[cells.z] << 16;
-        if (mask & 8u) tangent_axes |= (uint32_t)g.tangent_axes[cells.w] << 24;
-    }
+    // Along a tangent: the quad's cells' axes, a byte each, and their first factors.
+    const uint32_t tangent_axes = RECORD == kTangent ? g.quad_tangent_axes[q] : 0u;
+    const uint4 tangent_start = RECORD == kTangent ? g.quad_tangent_start[q] : make_uint4(0, 0, 0, 0);
     Quad<T> total{}, rise;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -919,21 +914,17 @@ __device__ __forceinline__ void step_layer(const Tables &g, const Fields<T> &f, 
             const T old_below = s.lo[a].v[j], old_above = s.hi[a].v[j], before = s.part[a].v[j];
             const T below = (T)c0.z * old_below - (T)c0.w * (here - lo);
             const T above = (T)c1.z * old_above - (T)c1.w * (hi - here);
-            if (recording && (mask & (1u << j))) {
-                const uint32_t own = j == 0 ? cells.x : (j == 1 ? cells.y : (j == 2 ? cells.z : cells.w));
-                const uint32_t cell = RECORD == kTangent ? own : g.lane_cell[4 * (uint64_t)q + j];
-                const uint32_t axes = RECORD == kTangent ? tangent_axes >> (8 * j) : g.tangent_axes[cell];
-                if (axes & (1u << a)) {
-                    // The step's factors along the tangent: its products with the adjoints of the new
-                    // part and faces give the gradient's step (fdtd_adjoint.cuh), in double.
-                    const uint32_t x0 = a == 0 ? x + j : at;
-                    const double2 tc = g.tangent_centre[a][x0];
-                    const double2 t0 = g.tangent_face[a][x0], t1 = g.tangent_face[a][x0 + 1];
-                    T *o = f.traj_tangent + g.tangent_start[cell] + 3 * __popc(axes & ((1u << a) - 1u));
-                    o[0] = (T)((double)before * tc.x - (double)sc.v[j] * (double)(above - below) * tc.y);
-                    o[1] = (T)((double)old_above * t1.x - (double)(hi - here) * t1.y);
-                    o[2] = (T)((double)old_below * t0.x - (double)(here - lo) * t0.y);
-                }
+            if (RECORD == kTangent && (tangent_axes >> (8 * j + a) & 1u)) {
+                // The step's factors along the tangent: its products with the adjoints of the new
+                // part and faces give the gradient's step (fdtd_adjoint.cuh), in double.
+                const uint32_t x0 = a == 0 ? x + j : at;
+                const double2 tc = g.tangent_centre[a][x0];
+                const double2 t0 = g.tangent_face[a][x0], t1 = g.tangent_face[a][x0 + 1];
+                const uint32_t start = j == 0 ? tangent_start.x : (j == 1 ? tangent_start.y : (j == 2 ? tangent_start.z : tangent_start.w));
+                T *o = f.traj_tangent + start + 3 * __popc((tangent_axes >> (8 * j)) & ((1u << a) - 1u));
+                o[0] = (T)((double)before * tc.x - (double)sc.v[j] * (double)(above - below) * tc.y);
+                o[1] = (T)((double)old_above * t1.x - (double)(hi - here) * t1.y);
+                o[2] = (T)((double)old_below * t0.x - (double)(here - lo) * t0.y);
             }
             rise.v[j] = above - below;
             const T push = SCALED ? (T)c0.y * sc.v[j] : (T)c0.y;

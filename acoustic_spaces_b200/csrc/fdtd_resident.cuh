@@ -35,8 +35,8 @@ struct ResidentArgs {
     T *gathered;
     uint32_t gathered_count;
     // Recording (Fields): the first step's places, or null.
-    T *traj_u, *traj_w, *traj_layer, *traj_tangent;
-    uint32_t states, tangent_factors;
+    T *traj_u, *traj_w, *traj_layer;
+    uint32_t states;
     uint32_t steps;
     uint32_t clustered;     // the launch is one cluster: its barrier in place of the counter
     unsigned int *arrived;  // blocks arrived at the steps' barriers so far
@@ -293,7 +293,6 @@ __global__ void __launch_bounds__(kResidentThreads<T, WIDE, LAYER>, 1)
         f.signal = p.signal + k;
         if (p.traj_u) f.traj_u = p.traj_u + (uint64_t)k * g.specials, f.traj_w = p.traj_w + (uint64_t)k * p.states;
         if (LAYER && p.traj_layer) f.traj_layer = p.traj_layer + (uint64_t)k * 18 * g.layer_lanes;
-        if (LAYER && p.traj_tangent) f.traj_tangent = p.traj_tangent + (uint64_t)k * p.tangent_factors;
         uint4 here = first;
         for (uint32_t t = warp; t < all; t += kWarps) {
             const uint4 e = here;
