@@ -333,7 +333,7 @@ __device__ __forceinline__ void layer_hat_cell(const AdjointTables &t, uint32_t 
 // The tables' products of `steps` steps whose Q^, L^, H^ waited (layer_hat_cell; step k's at waiting + 9 k
 // layers), with their forward factors: `traj` the first's, each next one's a step's factors before. The
 // steps' products are added in turn, one read and write of a cell's eighteen double sums for all of
-// them (their 288 bytes a cell are most of what a step of the tables' gradient moves). A row of blocks an
+// them (288 bytes a cell a step, were they read and written every step). A row of blocks an
 // axis.
 template <typename T, bool CELLS = false>
 __global__ void __launch_bounds__(kBlock) layer_pending_kernel(const AdjointTables t, const T *waiting, uint32_t steps,

@@ -1160,7 +1160,8 @@ bool gathers(const fdtd_layout *L, uint64_t e) {
 // Measured, us a step, launched (each kind on its stream) and resident, at so many air cells:
 //   FP32 boxes 0.58M 6.1 and 4.2, 1.5M 7.0 and 6.5, 2.6M 7.5 and 9.0, 8.6M 21.5 and 25.0; compensated 1.5M 7.4 and 7.3, 2.6M 8.7
 //   and 10.4; the wide stencil 0.86M 8.1 and 6.5, 1.7M 9.5 and 9.4, 3.5M 13.8 and 16.8;
-//   FP32 with a matched layer 0.34M (0.19M layer cells) 6.9 and 4.9, 0.68M 8.2 and 8.1, 1.3M 13.1 and 14.0-17.2;
+//   FP32 with a matched layer 0.34M (0.19M layer cells) 6.9 and 4.1, 0.68M 8.2 and 6.1, 1.3M 13.1 and 14.0-17.2 (with the
+//   code that records along a tangent still in the resident kernel, where 0.34M took 4.9 and 0.68M 8.1);
 //   double 1.5M 10.9 and 9.8, 2.6M 14.1 and 14.5, 4.3M 23.8 and 22.4, 8.6M 48.0 and 45.3, 10.8M 58.6 and 61.3; with a layer
 //   0.68M 12.6 and 11.5, 1.3M 24.6 and 20.2-23.3, 2.1M 37-44 and 36-45; wide 0.86M 10.9 and 10.5, 1.7M 14.6 and 16.1.
 bool takes_resident(const fdtd_solver *s, const fdtd_layout *L) {

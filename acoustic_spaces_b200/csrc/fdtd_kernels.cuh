@@ -982,7 +982,8 @@ __global__ void __launch_bounds__(kBlock, sizeof(T) == 4 ? 4 : 3) layer_kernel(c
 // Probe p's pressure before the step (fdtd.hpp:3525-3533): its cells' weighted sum in double, in
 // the layout's order. A warp per probe: the lanes load the cells and form the products (each
 // product is the reference's own), then lane 0 adds them up in the layout's order, so that the
-// sum rounds as the reference's sequential one. (Moving air, whose carry follows the record.)
+// sum rounds as the reference's sequential one. (Single steps, probes of more cells than are gathered, and moving
+// air, whose carry follows the record.)
 constexpr int kProbeWarps = kBlock / 32;
 
 template <typename T>
